@@ -272,211 +272,227 @@ __global__ void __launch_bounds__(T) k_tree(const SliceWork* __restrict__ work, 
 // ---------------------------------------------------------------------------
 // k_rlgr
 //
-// Bit window: 64 bits `hi:lo` of the stream with the next bit at bit `o`
-// (0..31, counted from the MSB) of `hi`: peek() returns the next 32 bits with
-// one funnel shift, advance(n <= 32) consumes n of them and takes the next
-// word into the window when `o` passes 32.  Words come from 16-byte payload
-// blocks staged in shared memory: each thread owns a ring of kRing block
-// slots (slot j of thread t at s_ring[j * blockDim + t], so a warp's 16-byte
-// reads are conflict-free), filled by cp.async kRing - 1 blocks -- about 75
-// loop iterations -- ahead of their use, so the serial chain does not wait
-// on global memory.  `cur` holds the words of the current block not yet
-// taken (the next one in cur.x).  Blocks past the payload are zero-filled.
-constexpr int kRing = 4;
-
-__device__ __forceinline__ void ring_fetch(uint4* slot, const uint4* src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(slot);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(valid ? 16 : 0) : "memory");
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-// every block but the kRing - 2 most recently requested has landed
-__device__ __forceinline__ void ring_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(kRing - 2) : "memory"); }
+// Bit window: two words `hi:lo` of the stream, complemented, with the next bit
+// at bit `o` (0..31, counted from the MSB) of `hi`, and the word after them,
+// `nx`, as loaded: the next 32 bits are one funnel shift away, and the load of
+// a word is issued when the one before it enters the window, a dozen
+// iterations ahead of its use.
+//
+// Words come from 16-byte payload blocks staged in shared memory: each lane
+// owns a ring of kRing blocks (kRing * 16 bytes, aligned to its size), filled
+// by cp.async.  The copies are requested at a point the whole warp passes
+// together (stage(), every kRlCheck iterations: as many blocks as those can
+// take),
+// never from inside a lane's own branch: with 32 slices in a warp, some lane
+// needs a block in nearly every iteration, and each such branch cost the warp
+// its instructions and a wait for copies that other lanes had just requested.  `landed` counts the blocks
+// known to be in shared memory: those requested three stage() calls ago.  A
+// lane that may run out of landed words before the next stage() -- only after
+// codes longer than 32 bits -- refills its ring synchronously.  Blocks past
+// the payload are zero.
+constexpr int kRing = 8;             // 16-byte blocks per lane
+constexpr uint32_t kRlCheck = 8;     // iterations between stage() calls (4: 5-10% slower, 16: no faster);
+                                     // a fast iteration takes at most one word
 
 struct BitReader {
-    const uint4* p;      // next block to request
-    const uint4* end;    // one past the last block holding payload bytes
     const uint4* first;  // the slice's first block
-    uint4* ring;         // this thread's slot 0
-    uint32_t stride;     // between slots (uint4 units)
-    uint32_t rb;         // blocks read from the ring
-    uint4 cur;
-    uint32_t ci;         // words left in cur
-    uint32_t hi, lo;
-    uint32_t o;
+    uint32_t nblk;       // blocks holding payload bytes
+    uint32_t ring;       // shared address of this lane's ring
+    uint32_t hi, lo, nx, o;
+    uint32_t wi;         // index of the word after nx
+    uint32_t sp;         // blocks requested
+    uint32_t s1, s2, s3;  // ... as of the last three stage() calls
+    uint32_t landed;     // blocks that have landed (at most kRing of them still in the ring)
 
-    __device__ __forceinline__ static uint32_t be(uint32_t w) { return __byte_perm(w, 0, 0x0123); }
-    __device__ __forceinline__ void request() {  // block p into the slot of the block read last
-        const bool valid = p < end;
-        ring_fetch(ring + ((rb + kRing - 1) & (kRing - 1)) * stride, valid ? p : first, valid);
-        ++p;
-    }
-    __device__ __forceinline__ uint4 next_block() {
-        ring_wait();
-        const uint4 v = ring[(rb & (kRing - 1)) * stride];
-        request();
-        ++rb;
+    __device__ __forceinline__ static uint32_t inv(uint32_t w) { return ~__byte_perm(w, 0, 0x0123); }
+    __device__ __forceinline__ uint32_t slot(uint32_t blk) const { return ring | ((blk << 4) & (kRing * 16 - 1)); }
+    __device__ __forceinline__ uint32_t ring_word(uint32_t w) const {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(ring | ((w << 2) & (kRing * 16 - 1))));
         return v;
     }
-    __device__ __forceinline__ void init(const uint8_t* payload, uint64_t off, uint32_t nbytes, uint4* ring0, uint32_t str) {
-        first = p = reinterpret_cast<const uint4*>(payload + (off & ~15ull));
-        end = reinterpret_cast<const uint4*>(payload + ((off + nbytes + 15) & ~15ull));
-        ring = ring0;
-        stride = str;
-        rb = 0;
-        for (int j = 0; j < kRing - 1; ++j) {  // blocks 0 .. kRing-2 into slots 0 .. kRing-2
-            const bool valid = p < end;
-            ring_fetch(ring + j * stride, valid ? p : first, valid);
-            ++p;
-        }
-        const uint4 b0 = next_block();
-        hi = be(b0.x);
-        lo = be(b0.y);
-        cur = make_uint4(b0.z, b0.w, 0u, 0u);
-        ci = 2;
-        o = 0;
-        uint32_t skip = (uint32_t)(off & 15) * 8;  // payload bytes before the slice's first byte
-        while (skip >= 32) {
-            advance(32);
-            skip -= 32;
-        }
-        advance(skip);
+    __device__ __forceinline__ uint32_t payload_word(uint32_t w) const {  // straight from the payload
+        return (w >> 2) < nblk ? __ldg(reinterpret_cast<const uint32_t*>(first) + w) : 0u;
     }
-    // the next 32 bits of the stream
-    __device__ __forceinline__ uint32_t peek() const { return __funnelshift_l(lo, hi, o); }
-    // consume n <= 32 bits; branch-free apart from the block refill (a lane
-    // needs one about every 25 iterations)
+    __device__ __forceinline__ uint32_t base_block() const { return (wi - 1) >> 2; }  // nx's: the first still read
+    __device__ __forceinline__ void request() {  // block sp into its slot
+        const bool valid = sp < nblk;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(slot(sp)), "l"(first + (valid ? sp : 0u)),
+                     "r"(valid ? 16 : 0)
+                     : "memory");
+        ++sp;
+    }
+    // every lane of the warp: the copies of three calls ago have landed; the
+    // blocks of kRlCheck more iterations requested
+    __device__ __forceinline__ void stage(bool active) {
+        asm volatile("cp.async.wait_group 2;\n" ::: "memory");
+        landed = s3;
+        s3 = s2;
+        s2 = s1;
+#pragma unroll
+        for (uint32_t j = 0; j < kRlCheck / 4; ++j)
+            if (active && sp < base_block() + kRing) request();
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        s1 = sp;
+    }
+    // the words up to the next stage() may not all have landed
+    __device__ __forceinline__ bool short_of_words() const { return 4 * landed < wi + kRlCheck; }
+    __device__ __forceinline__ void refill() {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        sp = max(sp, base_block());
+        for (; sp < base_block() + kRing; ++sp) {
+            const uint4 b = sp < nblk ? __ldg(first + sp) : make_uint4(0, 0, 0, 0);
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(slot(sp)), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                         : "memory");
+        }
+        s1 = s2 = s3 = landed = sp;
+    }
+    // a lane without a slice (it takes part in stage() only)
+    __device__ __forceinline__ void idle() {
+        first = nullptr;
+        nblk = ring = hi = lo = nx = o = wi = sp = s1 = s2 = s3 = landed = 0;
+    }
+    __device__ __forceinline__ void init(const uint8_t* payload, uint64_t off, uint32_t nbytes, uint4* ring0) {
+        first = reinterpret_cast<const uint4*>(payload + (off & ~15ull));
+        nblk = (uint32_t)((((uint64_t)(off & 15) + nbytes) + 15) >> 4);
+        ring = (uint32_t)__cvta_generic_to_shared(ring0);
+        const uint32_t w0 = (uint32_t)(off & 15) >> 2;  // payload words before the slice's first byte
+        hi = inv(payload_word(w0));
+        lo = inv(payload_word(w0 + 1));
+        nx = payload_word(w0 + 2);
+        wi = w0 + 3;
+        o = (uint32_t)(off & 3) * 8;
+        sp = base_block();
+        for (int j = 0; j < kRing; ++j) request();
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        s1 = s2 = s3 = landed = sp;
+    }
+    // the next 32 bits of the stream, complemented
+    __device__ __forceinline__ uint32_t peek_inv() const { return __funnelshift_l(lo, hi, o); }
+    __device__ __forceinline__ uint32_t peek() const { return ~peek_inv(); }
+    // consume n <= 32 bits, the words landed (fast iterations); n = 0: nothing
     __device__ __forceinline__ void advance(uint32_t n) {
         o += n;
         const bool take = o >= 32;
         o &= 31u;
         hi = take ? lo : hi;
-        lo = take ? be(cur.x) : lo;
-        cur.x = take ? cur.y : cur.x;
-        cur.y = take ? cur.z : cur.y;
-        cur.z = take ? cur.w : cur.z;
-        ci -= take ? 1u : 0u;
-        if (ci == 0) {
-            cur = next_block();
-            ci = 4;
+        lo = take ? inv(nx) : lo;
+        wi += take ? 1u : 0u;
+        nx = ring_word(wi - 1);
+    }
+    // consume n <= 32 bits, the words from the payload (outside the fast iterations)
+    __device__ __forceinline__ void advance_slow(uint32_t n) {
+        o += n;
+        if (o >= 32) {
+            hi = lo;
+            lo = inv(nx);
+            nx = payload_word(wi);
+            ++wi;
+            o &= 31u;
         }
     }
-    // payload bits consumed: the words that entered the window before hi,
-    // plus o, minus the bytes before the slice in its first block
+    // payload bits consumed: the words before hi plus o, minus the bytes
+    // before the slice in its first block
     __device__ __forceinline__ int64_t consumed(uint64_t off) const {
-        const int64_t words = (int64_t)rb * 4 - (int64_t)ci;  // entered the window
-        return (words - 2) * 32 + (int64_t)o - (int64_t)(off & 15) * 8;
+        return ((int64_t)wi - 3) * 32 + (int64_t)o - (int64_t)(off & 15) * 8;
     }
-    // no copy of this thread's left in flight (before its shared memory is reused)
+    // no copy of this thread's left in flight (before the CTA ends)
     __device__ __forceinline__ void drain() const { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 };
 
 constexpr uint32_t kRlU0 = 3, kRlU1 = 2, kRlD0 = 1, kRlD1 = 1, kRlMaxRP = 32 * 4;
 
-// Zero-run length of `c` leading ones read in run mode from state kP
-// (entropy_codec.cc:228-233): the i-th one stands for 2^((kP + 2i) >> 2)
-// zeros, kP growing by U1 = 2 per one, so the exponents go in pairs.  With
-// S(n) = sum_{i<n} 2^(i>>1) = 2 (2^(n>>1) - 1) + (n & 1) 2^(n>>1):
-//   kP & 3 in {0,1}:  sum = 2^(kP>>2) S(c)
-//   kP & 3 in {2,3}:  sum = 2^(kP>>2) (S(c+1) - 1)
-// Every term is below 2^k with k = (kP + 2c) >> 2, so when the whole run code
-// (c ones, a zero, k bits) fits 32 bits the length fits 32 bits too.
-__device__ __forceinline__ uint32_t run_ones_length(uint32_t kP, uint32_t c) {
-    const uint32_t hi = (kP >> 1) & 1u;  // exponent pairs start one late
-    const uint32_t n = c + hi;
-    const uint32_t h = 1u << (n >> 1);
-    const uint32_t S = 2 * (h - 1) + (n & 1u) * h - hi;
-    return S << (kP >> 2);
+// leading zeros of w; all ones (-1) for w = 0
+__device__ __forceinline__ uint32_t lead0(uint32_t w) {
+    uint32_t d;
+    asm("bfind.shiftamt.u32 %0, %1;" : "=r"(d) : "r"(w));
+    return d;
 }
 
-// bits [at, at + k) of w (k <= 32; k = 0 gives 0, and so does at >= 32)
-__device__ __forceinline__ uint32_t field(uint32_t w, uint32_t at, uint32_t k) {
-    return __funnelshift_rc(__funnelshift_lc(0u, w, at), 0u, 32u - k);
-}
-
-// k_rlgr: one thread per slice.  The coefficient planes are zeroed before the
-// launch, so a run of zeros only moves the output position; symbol j of a
-// plane goes to coefficient N-1-j (the stream is reversed).  The loop keeps
-// 32-bit state only: `dst` walks down the current plane, `rem` counts the
-// plane's symbols still to come, `left` all symbols still to come.
-//
-// One iteration = an optional zero run (run mode, kP >= 4) followed by one
-// Golomb-Rice symbol.  The common case -- run code and symbol code together
-// within the next 32 bits, a symbol below 2^23, the run inside the current
-// plane -- is one branch-free line that every lane of a warp executes in
+// One iteration of a slice's serial chain = an optional zero run (run mode,
+// kP >= 4) followed by one Golomb-Rice symbol.  RlFast evaluates it on the
+// next 32 bits in one branch-free line that every lane of a warp executes in
 // step, whatever mode its slice is in (a lane outside run mode computes an
-// empty run): the run's leading ones are counted with one clz and summed in
-// closed form (run_ones_length), the symbol's ones with a second clz on the
-// same 32 bits, and one advance consumes both.  Its dependent chain is about
-// fifteen integer operations.  All other iterations (longer codes, the
-// 32-ones escape, wide symbols, runs across a plane or to the end of the
-// slice) take the general path, which reads the codes piece by piece as the
-// reference does; at q = 8 about one lane-iteration in 4,000 goes there.
+// empty run): the leading ones of the run code by one bit search, its length
+// in closed form, the symbol's ones by a second bit search on the same bits,
+// and one advance consumes both.
 //
-// LANES < 32: only the first LANES lanes of each warp decode (the rest exit at
-// once), so a warp executes the union of fewer lanes' paths per iteration --
-// for the longest slices, whose serial chains set the kernel's length.
-template <int T, int LANES = 32>
-__global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, const int32_t* __restrict__ order,
-                                              int nslices, const uint8_t* __restrict__ payload, float* __restrict__ coef,
-                                              int32_t* __restrict__ rstatus) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if ((g & 31) >= LANES) return;
-    const int t = (g >> 5) * LANES + (g & 31);
-    if (t >= nslices) return;
-    const int item = order[t];
-    const SliceWork& wk = work[item];
-    const uint32_t N = wk.n;
-    const int32_t qp = wk.qp;
-    if (N == 0) {
-        rstatus[item] = PVVC_OK;
-        return;
-    }
-    const uint64_t off = wk.col_off;
-    const uint32_t csz = wk.csz;
-    extern __shared__ uint4 s_ring[];  // kRing * blockDim payload blocks
-    BitReader br;
-    br.init(payload, off, csz, s_ring + threadIdx.x, blockDim.x);
-    const uint32_t csh = wk.coef_stride == 32 ? 5u : 0u;   // coefficient stride 32 (group region) or 1
-    const int64_t cs = (int64_t)1 << csh;
-    const int64_t wrap = (int64_t)(2 * N - 1) << csh;       // last coefficient of a plane -> top of the next
-    float* dst = coef + wk.coef_off + ((uint64_t)(N - 1) << csh) + wk.coef_lane;  // coefficient of the next symbol
-    uint32_t rem = N;                         // symbols left in the current plane
-    uint32_t left = 3u * N;                   // symbols left in the slice
-    uint32_t kP = 0, kRP = 8;
-    int err = PVVC_OK;
-    for (;;) {
-        // ---- common case: the whole iteration within the next 32 bits ----
-        const uint32_t v = br.peek();
+// Run length.  c ones read in run mode from state kP stand for
+// sum_{i<c} 2^((kP + 2i) >> 2) zeros (entropy_codec.cc:228-233; kP grows by
+// U1 = 2 per one).  With G(t) = (2 | (t & 1)) << (t >> 1), and t = kP >> 1
+// before and t2 = t + c after the ones, that sum is G(t2) - G(t); k = t2 >> 1
+// remainder bits follow.  Let z be the complemented bits of the zero and the
+// remainder read together (k + 1 bits): the remainder is 2^(k+1) - 1 - z, and
+// run + 1 = ((4 | (t2 & 1)) << k) - z - G(t).
+//
+// Symbol.  q ones, a zero and kR bits: with z the complemented zero and
+// remainder, u = ((q + 2) << kR) - 1 - z.
+//
+// The iteration is fast when the codes lie within the 32 bits, kRP is small
+// (kR <= 17, so that the symbol is below 2^23, and kRP + q - 1 needs no cap)
+// and run + 1 <= left.  32 leading ones make c or q all ones: then r + q is
+// either 32 or all ones, and the test fails.  Everything else (longer codes,
+// the 32-ones escape, wide symbols) goes to RlSlow, about one lane-iteration
+// in 4,000 at q = 8.
+//
+// kRlCheck iterations run without a branch: a lane whose iteration is not
+// fast changes nothing until the check that follows them, so the compiler
+// schedules one iteration's stores and adaptation into the next one's chain.
+// What bounds the kernels is that chain and the ~80 instructions of an
+// iteration on one or two warps per scheduler.  Longest slices of a GoP of 30
+// frames of 800k points (8,200 iterations, 15 CTAs): 1.51 ms with the refills
+// and the general path inside the loop, 0.96 ms now; windowed larger half of
+// the medium tier 1.10 -> 0.59 ms, shorter half 0.75 -> 0.41, short tier
+// 0.57 -> 0.34.
+constexpr uint32_t kRlFastRP = 72;
+struct RlFast {
+    uint32_t kPn, kRPn, bits, m1, zz;
+    bool ok;
+    __device__ __forceinline__ RlFast(uint32_t vi, uint32_t kP, uint32_t kRP, uint32_t left) {
         const bool run = kP >= 4;
-        const uint32_t c = run ? __clz(~v) : 0u;   // leading ones of the run code
-        const uint32_t kP2 = kP + 2 * c;           // kP after the ones
-        const uint32_t k = run ? (kP2 >> 2) : 0u;  // remainder bits of the run code
-        const uint32_t r = run ? c + 1 + k : 0u;   // bits of the run code
-        const uint32_t v2 = __funnelshift_lc(0u, v, r);  // the symbol's code, left-aligned
-        const uint32_t q = __clz(~v2);             // its leading ones
-        const uint32_t kR = kRP >> 2;
-        const uint32_t nb = r + q + 1 + kR;        // bits of the whole iteration
-        const uint32_t u = (q << kR) | field(v2, q + 1, kR);
-        const uint32_t m = run ? run_ones_length(kP, c) + field(v, c + 1, k) : 0u;  // zeros of the run
-        if (nb <= 32 && u < (1u << 23) && m < rem) {
-            br.advance(nb);
-            dst -= (int64_t)m << csh;
-            const uint32_t zz = u + (uint32_t)run;  // Unsign2Sign(u + after_run) * qp, stored unless zero
-            const int32_t sym = (int32_t)(zz >> 1) ^ -(int32_t)(zz & 1);
-            if (sym) *dst = __int2float_rn(sym * qp);
-            // adaptation (entropy_codec.cc:245-281); here p = u >> kR = q
-            kRP = q ? min(kRP + q - 1, kRlMaxRP) : (kRP < 2 ? 0u : kRP - 2);
-            kP = (run || u) ? (kP2 ? kP2 - kRlD1 : 0u) : kP2 + kRlU0;  // D0 = D1 = 1
-            left -= m + 1;
-            rem -= m + 1;
-            const bool end_of_plane = rem == 0;
-            dst += end_of_plane ? wrap : -cs;
-            rem = end_of_plane ? N : rem;
-            if (left == 0) break;
-            continue;
-        }
-        // ---- general path: the codes read piece by piece ----
-        uint32_t mm = 0;   // zeros in the run
+        const uint32_t nrun = run ? 0u : 0xFFFFFFFFu;
+        const uint32_t c = lead0(vi | nrun);
+        const uint32_t kP2 = kP + 2 * c;
+        const uint32_t k = kP2 >> 2;
+        const uint32_t r = c + k + (nrun + 1u);  // bits of the run code
+        const uint32_t w = __funnelshift_lc(0xFFFFFFFFu, vi, r);
+        const uint32_t q = lead0(w);
+        const uint32_t kR = kRP >> 2, nR = 31u - kR, rq = r + q;
+        bits = rq + (kR + 1u);
+        const uint32_t G = (2u | ((kP >> 1) & 1u)) << (kP >> 2);
+        const uint32_t z0 = __funnelshift_r(__funnelshift_l(0u, vi, c), 0u, ~k);  // >> 31 - k
+        m1 = run ? (__funnelshift_l(0u, 4u | ((kP2 >> 1) & 1u), k) - z0 - G) : 1u;
+        const uint32_t z1 = __funnelshift_r(__funnelshift_l(0u, w, q), 0u, nR);
+        zz = __funnelshift_l(0u, q + 2u, kR) - z1 + nrun;  // u + run
+        // outside run mode u = 0 when the zero and the remainder are all zeros
+        const bool zero = !run && vi >= __funnelshift_l(0u, 0xFFFFFFFFu, nR);
+        ok = rq <= nR && kRP < kRlFastRP && m1 <= left;
+        // adaptation (entropy_codec.cc:245-281); here p = u >> kR = q
+        kRPn = q ? kRP + q - 1u : max(kRP, 2u) - 2u;
+        kPn = zero ? kP2 + kRlU0 : max(kP2, 1u) - 1u;  // D0 = D1 = 1
+    }
+    // float(Unsign2Sign(zz) * qp): x = ceil(zz / 2) is below 2^23 here (zz <=
+    // 15 << 17), so it is the low mantissa of 2^23 + x and needs no conversion;
+    // the float product rounds the exact one once, as the conversion of the
+    // integer product does.  zz odd is negative (sign: 2^31, or 0 for qp = 0,
+    // whose products are +0).
+    __device__ __forceinline__ float value(float qp, uint32_t sign) const {
+        const float x = __fmul_rn(__fsub_rn(__uint_as_float(0x4B000000u + ((zz + 1u) >> 1)), 8388608.0f), qp);
+        return __uint_as_float(__float_as_uint(x) ^ ((zz << 31) & sign));
+    }
+};
+
+// One iteration read piece by piece, as the reference does.  `left`: symbols
+// of the slice still to come.  The run's zeros (at most `left`) in m; a symbol
+// follows unless they end the slice or the code is malformed (err).
+struct RlSlow {
+    uint32_t m = 0;
+    long long sym = 0;
+    bool has = false;
+    int err = PVVC_OK;
+    __device__ __forceinline__ RlSlow(BitReader& br, uint32_t& kP, uint32_t& kRP, uint32_t left) {
+        const bool run = kP >= 4;
         uint32_t kPr = kP;  // kP after the run's ones
         if (run) {
             // zero run (entropy_codec.cc:226-233): ones, a zero, k remainder bits
@@ -485,54 +501,42 @@ __global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, 
             uint32_t cc;
             int guard = 0;
             do {
-                cc = __clz(~br.peek());
+                cc = __clz(br.peek_inv());
                 for (uint32_t i = 0; i < cc; ++i) {
                     m64 += 1ull << (kk & 31);
                     kPr += kRlU1;
                     kk = kPr >> 2;
                 }
-                br.advance(cc);
+                br.advance_slow(cc);
             } while (cc == 32 && ++guard < 64);
-            br.advance(1);
+            br.advance_slow(1);
             if (kk > 31) {
                 err = PVVC_ERR_OVERRUN;
-                break;
+                return;
             }
-            m64 += br.peek() >> (32 - kk);
-            br.advance(kk);
-            mm = m64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)m64;
+            m64 += kk ? br.peek() >> (32 - kk) : 0u;
+            br.advance_slow(kk);
+            m = m64 > left ? left : (uint32_t)m64;
+            if (m == left) return;
         }
-        // skip mm zeros (they may cross plane boundaries)
-        {
-            uint32_t z = mm < left ? mm : left;
-            left -= z;
-            while (z >= rem && rem) {
-                z -= rem;
-                dst += (int64_t)(2 * N - rem) << csh;  // to the top of the next plane
-                rem = N;
-            }
-            dst -= (int64_t)z << csh;
-            rem -= z;
-        }
-        if (left == 0) break;
         // Golomb-Rice symbol (GRRead, entropy_codec.cc:196-205)
-        const uint32_t w = br.peek();
-        const uint32_t qq = __clz(~w);
+        const uint32_t kR = kRP >> 2;
+        const uint32_t qq = __clz(br.peek_inv());
         uint64_t uw;
         uint32_t pq;
         if (qq < 32) {
-            br.advance(qq + 1);
+            br.advance_slow(qq + 1);
             uint32_t rr = 0;
             if (kR) {
                 rr = kR >= 32 ? br.peek() : (br.peek() >> (32 - kR));
-                br.advance(kR >= 32 ? 32u : kR);
+                br.advance_slow(kR >= 32 ? 32u : kR);
             }
             uw = ((uint64_t)qq << kR) | rr;
             pq = qq;
         } else {  // 32 ones: a raw 32-bit value follows
-            br.advance(32);
+            br.advance_slow(32);
             const uint32_t raw = br.peek();
-            br.advance(32);
+            br.advance_slow(32);
             uw = raw;
             // p may be far above the kRP cap; any p > kRlMaxRP saturates
             // kRP + p - 1 at the cap (kRP >= 0), so clamp p to kRlMaxRP + 1,
@@ -542,23 +546,118 @@ __global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, 
         }
         kRP = pq ? min(kRP + pq - 1, kRlMaxRP) : (kRP < 2 ? 0u : kRP - 2);
         kP = (run || uw) ? (kPr ? kPr - kRlD1 : 0u) : kPr + kRlU0;
-        {
-            const uint64_t zz = uw + (uint64_t)run;
-            const long long sym = (long long)(zz >> 1) ^ -(long long)(zz & 1);
-            if (sym) *dst = __ll2float_rn(sym * (long long)qp);
-        }
-        --left;
-        const bool end_of_plane = --rem == 0;
-        dst += end_of_plane ? wrap : -cs;
-        rem = end_of_plane ? N : rem;
-        if (left == 0) break;
+        const uint64_t z = uw + (uint64_t)run;
+        sym = (long long)(z >> 1) ^ -(long long)(z & 1);
+        has = true;
     }
-    // bits consumed vs the payload (the reference reads past it, which is undefined)
-    if (!err) {
-        if (br.consumed(off) > 8ll * csz) err = PVVC_ERR_OVERRUN;
+};
+
+__device__ __forceinline__ void st_if(float* p, float v, bool c) {  // *p = v where c, without a branch
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.global.f32 [%0], %1;\n}\n" ::"l"(p), "f"(v),
+                 "r"((uint32_t)c)
+                 : "memory");
+}
+__device__ __forceinline__ void st_shared_if(uint32_t a, float v, bool c) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\n@p st.shared.f32 [%0], %1;\n}\n" ::"r"(a), "f"(v),
+                 "r"((uint32_t)c)
+                 : "memory");
+}
+
+// k_rlgr: one thread per slice.  The coefficient planes are zeroed before the
+// launch, so a run of zeros only moves the output position; symbol j of a
+// plane goes to coefficient N-1-j (the stream is reversed), which is also the
+// number of the plane's symbols still to come after it.
+//
+// LANES < 32: only the first LANES lanes of each warp decode, so a warp
+// executes the union of fewer lanes' paths per iteration.
+template <int T, int LANES = 32>
+__global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, const int32_t* __restrict__ order,
+                                              int nslices, const uint8_t* __restrict__ payload, float* __restrict__ coef,
+                                              int32_t* __restrict__ rstatus) {
+    extern __shared__ __align__(128) uint4 s_ring[];  // kRing blocks per thread
+    const int lane = threadIdx.x & 31;
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (g >> 5) * LANES + lane;
+    BitReader br;
+    br.idle();
+    uint32_t N = 0, rem = 0;   // symbols of a plane; left in the current plane
+    uint32_t qp = 0;
+    int plane = 0;
+    int32_t item = -1;         // -1: no slice, or done
+    uint32_t kP = 0, kRP = 8;
+    float* dst = nullptr;      // the current plane
+    uint32_t stride = 0;
+    if (lane < LANES && t < nslices) {
+        const int it = order[t];
+        const SliceWork& wk = work[it];
+        N = rem = wk.n;
+        qp = wk.qp;
+        dst = coef + wk.coef_off + wk.coef_lane;
+        stride = wk.coef_stride;
+        if (N == 0) rstatus[it] = PVVC_OK;
+        else br.init(payload, wk.col_off, wk.csz, s_ring + threadIdx.x * kRing);
+        if (N != 0) item = it;
+    }
+    auto finish = [&](int err) {
+        const SliceWork& wk = work[item];
+        // bits consumed vs the payload (the reference reads past it, which is undefined)
+        if (!err && br.consumed(wk.col_off) > 8ll * wk.csz) err = PVVC_ERR_OVERRUN;
+        rstatus[item] = err;
+        rem = 0;
+        item = -1;
+    };
+    auto next_plane = [&]() {
+        if (plane == 2) {
+            finish(PVVC_OK);
+        } else {
+            ++plane;
+            dst += (uint64_t)N * stride;
+            rem = N;
+        }
+    };
+    const uint32_t sign = qp ? 0x80000000u : 0u;
+    const float fqp = (float)qp;
+    while (__any_sync(0xffffffffu, rem != 0)) {
+        bool ok = true;
+#pragma unroll
+        for (uint32_t it = 0; it < kRlCheck; ++it) {
+            const RlFast f(br.peek_inv(), kP, kRP, rem);
+            ok = f.ok;  // a lane that is not stays where it is until the check below
+            br.advance(ok ? f.bits : 0u);
+            kP = ok ? f.kPn : kP;
+            kRP = ok ? f.kRPn : kRP;
+            rem -= ok ? f.m1 : 0u;
+            st_if(dst + (uint64_t)rem * stride, f.value(fqp, sign), ok && f.zz != 0);
+        }
+        if (rem == 0 && item >= 0) next_plane();
+        // general iterations until the next one is fast (a slice's first
+        // coefficients, large ones, take some forty in a row)
+        while (!ok && rem != 0) {
+            ok = RlFast(br.peek_inv(), kP, kRP, rem).ok;
+            if (ok) break;
+            const RlSlow w(br, kP, kRP, rem + (uint32_t)(2 - plane) * N);
+            if (w.err) {
+                finish(w.err);
+            } else {
+                uint32_t z = w.m;  // zeros, possibly across planes
+                while (rem != 0 && z >= rem) {
+                    z -= rem;
+                    rem = 0;
+                    next_plane();
+                }
+                rem -= z;
+                if (w.has) {
+                    --rem;
+                    if (w.sym) dst[(uint64_t)rem * stride] = __ll2float_rn(w.sym * (long long)(int32_t)qp);
+                    if (rem == 0) next_plane();
+                }
+            }
+        }
+        br.stage(rem != 0);
+        if (rem != 0 && br.short_of_words()) br.refill();
+        __syncwarp();
     }
     br.drain();
-    rstatus[item] = err;
 }
 
 // ---------------------------------------------------------------------------
@@ -571,7 +670,7 @@ __global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, 
 // Instead of scattered 4-byte stores into planes cleared beforehand, each
 // lane stages its nonzero symbols in a shared-memory window of WROWS rows
 // (row r = stream position r: the 32 lanes' words of that line, their eight
-// 16-byte chunks XOR-swizzled by r & 7).  Every kWinCheck iterations the
+// 16-byte chunks XOR-swizzled by r & 7).  Every kRlCheck iterations the
 // warp takes the smallest position any lane can still write
 // (__reduce_min_sync); rows below it are final for every lane.  Each full
 // unit of 32 final rows is written out with lane l taking row unit + l:
@@ -587,7 +686,6 @@ __global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, 
 // paused lane's position is at least WROWS rows ahead of the window, so the
 // minimum has passed a whole unit), so the loop ends after at most 3N rounds
 // per lane plus one flush per unit of rows.
-constexpr uint32_t kWinCheck = 4;        // iterations between window checks (a multiple of 2)
 constexpr uint32_t kWinUnit = 32;        // rows written out together (one per lane)
 constexpr int kWinRows = 64;             // window rows (8 KB per warp)
 
@@ -607,7 +705,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rlgr_win(const SliceWork* __rest
                                                          const uint8_t* __restrict__ payload, float* __restrict__ coef,
                                                          int32_t* __restrict__ rstatus) {
     static_assert((WROWS & (WROWS - 1)) == 0 && WROWS >= 2 * (int)kWinUnit, "window rows: a power of two");
-    extern __shared__ uint4 s_dyn[];  // [kRing][blockDim] payload blocks, then [WARPS][WROWS][32] floats
+    extern __shared__ __align__(128) uint4 s_dyn[];  // [blockDim][kRing] payload blocks, then [WARPS][WROWS][32] floats
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int gi = blockIdx.x * WARPS + wid;
     if (gi >= ngroups) return;  // the whole warp
@@ -623,11 +721,10 @@ __global__ void __launch_bounds__(32 * WARPS) k_rlgr_win(const SliceWork* __rest
     for (int i = lane; i < WROWS * 8; i += 32) reinterpret_cast<float4*>(win)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();  // rows are cleared by all lanes, then written by their owners
     BitReader br;
-    bool done = true, pend = false;
-    int err = PVVC_OK;
-    int32_t qp = 0;
-    uint64_t off = 0;
-    uint32_t csz = 0;
+    br.idle();
+    bool live = false, pend = false;
+    uint32_t qp = 0;
+    uint32_t s = total;             // stream position of this lane's next symbol (total: done)
     if (item >= 0) {
         const SliceWork& wk = work[item];
         if (wk.n != N) {
@@ -636,133 +733,91 @@ __global__ void __launch_bounds__(32 * WARPS) k_rlgr_win(const SliceWork* __rest
             rstatus[item] = PVVC_OK;
         } else {
             qp = wk.qp;
-            off = wk.col_off;
-            csz = wk.csz;
-            br.init(payload, off, csz, s_dyn + threadIdx.x, blockDim.x);
-            done = false;
+            br.init(payload, wk.col_off, wk.csz, s_dyn + threadIdx.x * kRing);
+            s = 0;
+            live = true;
         }
     }
-    uint32_t s = 0;                 // stream position of this lane's next symbol
+    auto finish = [&](int err) {
+        const SliceWork& wk = work[item];
+        // bits consumed vs the payload (the reference reads past it, which is undefined)
+        if (!err && br.consumed(wk.col_off) > 8ll * wk.csz) err = PVVC_ERR_OVERRUN;
+        rstatus[item] = err;
+        s = total;
+        live = false;
+    };
+    const uint32_t sign = qp ? 0x80000000u : 0u;
+    const float fqp = (float)qp;
+    const uint32_t win0 = (uint32_t)__cvta_generic_to_shared(win);
     uint32_t kP = 0, kRP = 8;
     uint32_t pend_q = 0;            // a pending symbol's position and value
     float pend_v = 0.f;
     uint32_t base = 0;              // rows below `base` are written out (warp-uniform)
     uint32_t bp = 0, bc = N - 1;    // plane and coefficient index of row `base`
-    for (uint32_t it = 1;; ++it) {
-        if (!done && !pend) {
-            uint32_t q = 0xFFFFFFFFu;  // position of a nonzero symbol decoded in this iteration
+    for (;;) {
+        // rows this lane may fill before the next check: to the end of the
+        // slice or of the window, none with a symbol pending
+        const uint32_t lim = min(total, base + (uint32_t)WROWS);
+        uint32_t room = pend || s >= lim ? 0u : lim - s;
+        const uint32_t end = s + room;
+        bool ok = true;
+#pragma unroll
+        for (uint32_t it = 0; it < kRlCheck; ++it) {
+            const RlFast f(br.peek_inv(), kP, kRP, room);
+            ok = f.ok;  // a lane that is not stays where it is until the check below
+            br.advance(ok ? f.bits : 0u);
+            kP = ok ? f.kPn : kP;
+            kRP = ok ? f.kRPn : kRP;
+            room -= ok ? f.m1 : 0u;
+            st_shared_if(win0 + 4u * slot(end - room - 1u), f.value(fqp, sign), ok && f.zz != 0);
+        }
+        s = end - room;
+        while (!ok && s < total && !pend) {
+            // a symbol beyond the window (it stays pending), or general
+            // iterations until the next one is fast
             float val = 0.f;
-            // ---- common case: the whole iteration within the next 32 bits ----
-            const uint32_t v = br.peek();
-            const bool run = kP >= 4;
-            const uint32_t c = run ? __clz(~v) : 0u;
-            const uint32_t kP2 = kP + 2 * c;
-            const uint32_t k = run ? (kP2 >> 2) : 0u;
-            const uint32_t r = run ? c + 1 + k : 0u;
-            const uint32_t v2 = __funnelshift_lc(0u, v, r);
-            const uint32_t qq = __clz(~v2);
-            const uint32_t kR = kRP >> 2;
-            const uint32_t nb = r + qq + 1 + kR;
-            const uint32_t u = (qq << kR) | field(v2, qq + 1, kR);
-            const uint32_t m = run ? run_ones_length(kP, c) + field(v, c + 1, k) : 0u;
-            if (nb <= 32 && u < (1u << 23) && m < total - s) {
-                br.advance(nb);
-                const uint32_t zz = u + (uint32_t)run;
-                const int32_t sym = (int32_t)(zz >> 1) ^ -(int32_t)(zz & 1);
-                if (sym) {
-                    q = s + m;
-                    val = __int2float_rn(sym * qp);
-                }
-                kRP = qq ? min(kRP + qq - 1, kRlMaxRP) : (kRP < 2 ? 0u : kRP - 2);
-                kP = (run || u) ? (kP2 ? kP2 - kRlD1 : 0u) : kP2 + kRlU0;
-                s += m + 1;
+            bool has = false;
+            const RlFast f(br.peek_inv(), kP, kRP, total - s);
+            ok = f.ok;
+            if (ok) {
+                if (s + f.m1 <= lim) break;
+                br.advance_slow(f.bits);
+                kP = f.kPn;
+                kRP = f.kRPn;
+                s += f.m1;
+                has = f.zz != 0;
+                val = f.value(fqp, sign);
             } else {
-                // ---- general path: the codes read piece by piece ----
-                uint32_t mm = 0, kPr = kP;
-                if (run) {
-                    uint64_t m64 = 0;
-                    uint32_t kk = kP >> 2;
-                    uint32_t cc;
-                    int guard = 0;
-                    do {
-                        cc = __clz(~br.peek());
-                        for (uint32_t i = 0; i < cc; ++i) {
-                            m64 += 1ull << (kk & 31);
-                            kPr += kRlU1;
-                            kk = kPr >> 2;
-                        }
-                        br.advance(cc);
-                    } while (cc == 32 && ++guard < 64);
-                    br.advance(1);
-                    if (kk > 31) {
-                        err = PVVC_ERR_OVERRUN;
-                    } else {
-                        m64 += br.peek() >> (32 - kk);
-                        br.advance(kk);
-                        mm = m64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)m64;
-                    }
-                }
-                if (!err) {
-                    s += min(mm, total - s);  // zeros, possibly across planes
-                    if (s < total) {
-                        const uint32_t w = br.peek();
-                        const uint32_t qw = __clz(~w);
-                        uint64_t uw;
-                        uint32_t pw;
-                        if (qw < 32) {
-                            br.advance(qw + 1);
-                            uint32_t rr = 0;
-                            if (kR) {
-                                rr = kR >= 32 ? br.peek() : (br.peek() >> (32 - kR));
-                                br.advance(kR >= 32 ? 32u : kR);
-                            }
-                            uw = ((uint64_t)qw << kR) | rr;
-                            pw = qw;
-                        } else {  // 32 ones: a raw 32-bit value follows (see k_rlgr on the clamp)
-                            br.advance(32);
-                            const uint32_t raw = br.peek();
-                            br.advance(32);
-                            uw = raw;
-                            const uint32_t t2 = kR >= 32 ? 0u : (raw >> kR);
-                            pw = t2 > kRlMaxRP ? kRlMaxRP + 1 : t2;
-                        }
-                        kRP = pw ? min(kRP + pw - 1, kRlMaxRP) : (kRP < 2 ? 0u : kRP - 2);
-                        kP = (run || uw) ? (kPr ? kPr - kRlD1 : 0u) : kPr + kRlU0;
-                        const uint64_t zz = uw + (uint64_t)run;
-                        const long long sym = (long long)(zz >> 1) ^ -(long long)(zz & 1);
-                        if (sym) {
-                            q = s;
-                            val = __ll2float_rn(sym * (long long)qp);
-                        }
-                        ++s;
-                    }
+                const RlSlow w(br, kP, kRP, total - s);
+                if (w.err) {
+                    finish(w.err);
+                } else {
+                    s += w.m + (uint32_t)w.has;
+                    has = w.sym != 0;
+                    val = __ll2float_rn(w.sym * (long long)(int32_t)qp);
                 }
             }
-            if (q != 0xFFFFFFFFu) {
-                if (q - base < (uint32_t)WROWS) {
-                    win[slot(q)] = val;
+            if (has) {
+                if (s - 1u - base < (uint32_t)WROWS) {
+                    win[slot(s - 1u)] = val;
                 } else {
                     pend = true;
-                    pend_q = q;
+                    pend_q = s - 1u;
                     pend_v = val;
                 }
             }
-            if (err || s >= total) {
-                done = true;
-                // bits consumed vs the payload (the reference reads past it, which is undefined)
-                if (!err && br.consumed(off) > 8ll * csz) err = PVVC_ERR_OVERRUN;
-                br.drain();
-                rstatus[item] = err;
-            }
         }
-        if (it % kWinCheck) continue;
+        if (live && s >= total) finish(PVVC_OK);
+        br.stage(live);
+        if (live && br.short_of_words()) br.refill();
+        __syncwarp();
         // ---- the window (warp-uniform) ----
-        const uint32_t lb = pend ? pend_q : (done ? total : s);  // this lane writes no row below lb
+        const uint32_t lb = pend ? pend_q : s;  // this lane writes no row below lb
         const uint32_t mn = __reduce_min_sync(0xffffffffu, lb);
         if (mn - base < kWinUnit && mn < total) continue;
         // write out whole units of final rows (and at the end the last,
         // partial one); rows from base + WROWS on were never staged: zeros
-        const uint32_t lim = base + WROWS;
+        const uint32_t top = base + WROWS;
         const uint32_t stop = mn == total ? total : base + (mn - base) / kWinUnit * kWinUnit;
         __syncwarp();  // every lane's staged words are visible to the row's owner
         while (base < stop) {
@@ -778,7 +833,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rlgr_win(const SliceWork* __rest
                 }
                 c -= d;
                 float4* dst = reinterpret_cast<float4*>(coef + region + (((uint64_t)p * N + c) << 5));
-                if (r < lim) {
+                if (r < top) {
                     float4* row = reinterpret_cast<float4*>(win + ((r & (WROWS - 1)) << 5));
 #pragma unroll
                     for (uint32_t j = 0; j < 8; ++j) {
