@@ -9,7 +9,7 @@
 //              164-184) level by level, the coded high-pass coefficients
 //              quantised (src/patch/GoP_encoding.cc:184-189) into the
 //              slice's symbol planes in stream (reversed) order
-//   k_rlgr_enc one thread per slice: RLGREncoder::Encode/GetResult
+//   k_rlgr_enc one CTA per group: RLGREncoder::Encode/GetResult
 //              (src/common/entropy_codec.cc:65-159) into the caller's buffer
 //
 // Bit-exactness with the CPU encoder: the butterfly pairs come from k_tree
@@ -28,7 +28,9 @@
 namespace pvvc {
 namespace {
 
-constexpr int kEncWarps = 8;
+// warps of a k_fwd_raht CTA; one CTA runs per SM (113 groups of 30 frames, 6M
+// points: 0.85 ms with 8 warps, 0.41 with 32)
+constexpr int kEncWarps = 32;
 
 __device__ __forceinline__ constexpr int epair0(int i) {
     return i == 1 ? 2 : i == 2 ? 4 : i == 3 ? 5 : i == 4 ? 8 : i == 5 ? 9 : i == 6 ? 10 : 11;
@@ -175,182 +177,335 @@ __global__ void __launch_bounds__(32 * kEncWarps) k_fwd_raht(const SliceWork* __
     }
 }
 
-// RLGREncoder: MSB-first bit writer over a 64-bit accumulator with the
-// reference's '+' (a value wider than its field would carry into the pending
-// bits before it; every caller here passes v < 2^bits, since the symbols are
-// int32), emitted as big-endian 32-bit words in order.
-struct BitSink {
-    uint32_t* out;       // 4-byte aligned region
-    uint32_t cap;        // bytes
-    uint32_t nwords = 0; // whole 32-bit words emitted
-    uint32_t nbytes = 0; // set by finish()
-    uint64_t acc = 0;    // pending bits in the low n bits
-    int n = 0;           // < 32 between calls
-    bool overflow = false;
-    __device__ __forceinline__ void emit(uint32_t w) {
-        if (++nwords * 4u <= cap) out[nwords - 1] = __byte_perm(w, 0, 0x0123);
-        else overflow = true;
-    }
-    __device__ __forceinline__ void put(uint64_t v, int bits) {
-        if (bits > 32) {
-            put(v >> 32, bits - 32);
-            put(v & 0xFFFFFFFFull, 32);
-            return;
-        }
-        acc = (acc << bits) + v;
-        n += bits;
-        if (n >= 32) {
-            n -= 32;
-            emit((uint32_t)(acc >> n));
-        }
-    }
-    __device__ __forceinline__ void gr(uint64_t x, int k) {  // GRWrite
-        const uint64_t p = x >> k;
-        if (p < 32) {
-            put((1ull << (p + 1)) - 2, (int)p + 1);  // p ones and a zero
-            put(x & ((1ull << k) - 1), k);
-        } else {
-            put(0xFFFFFFFFull, 32);
-            put(x, 32);
-        }
-    }
-    __device__ __forceinline__ void finish() {  // zero bits up to the byte boundary
-        nbytes = nwords * 4u + (uint32_t)((n + 7) >> 3);
-        if (n) {
-            const uint32_t w = (uint32_t)(acc << (32 - n));
-            if (nbytes <= cap) out[nwords] = __byte_perm(w, 0, 0x0123);
-            else overflow = true;
-        }
-    }
+constexpr uint32_t kU0 = 3, kU1 = 2, kMaxRP = 32 * 4;
+
+// k_rlgr_enc: RLGREncoder::Encode/GetResult, one CTA per group of slices (the
+// frames of one patch, all of N points), 64 symbols of every slice at a time.
+//
+// Only the adaptive state (kP, kRP, and m, the zeros of the unfinished run) is
+// serial.  Warp 0 steps it, lane f for slice f, branch-free, and leaves the
+// state each symbol sees in shared memory.  The other warps turn the chunk
+// before into bits meanwhile: a warp takes a slice, each lane builds the codes
+// of its two symbols from the states, a warp scan places them, and they are
+// ORed into the slice's bit buffer, whose full words go out.  The symbols of
+// the chunk after come in by cp.async; one barrier per chunk.  A lane's two
+// codes fit 32 bits nearly always; a slice's chunk where some lane's do not is
+// coded 32 symbols at a time in 64 bits.
+//
+// What bounds it is warp 0, about 35 instructions and 80 cycles a symbol, over
+// the longest slices.  3,390 slices of 18M symbols (longest 21,500): 11.0 ms as
+// a thread per slice in divergent 64-bit code, 1.79 ms as a warp per slice that
+// stepped its own state in every lane, 0.96 ms in this form (1.01 with 6 coders
+// instead of 12).
+constexpr int kEncWarpsR = 16;                // warp 0, three idle ones and the coders
+constexpr int kEncCoders = kEncWarpsR / 4 * 3;
+constexpr uint32_t kEncChunk = 64;            // symbols of a slice in a chunk, two per lane of its coder
+// Symbol j of slice f at word j * kEncRow + f: a row's lanes hit 32 banks, a
+// column's (a coder's lanes, two symbols apart) 16, and the stepper's addresses
+// are one register plus constants.
+constexpr uint32_t kEncRow = 33;
+__device__ __forceinline__ uint32_t enc_at(uint32_t j, uint32_t f) { return j * kEncRow + f; }
+// A symbol's state in one word, kP | kRP << 8 | (m & 0xFFFF) << 16.  m is below
+// 2^(kP >> 2), and kP rises by at most 2 per 2^(kP >> 2) zeros in run mode: from
+// below kEncWideP it stays below 68 for a chunk, so m's high half is zero.  A
+// chunk that a slice enters above it keeps the high halves in a second array.
+constexpr uint32_t kEncWideP = 60;
+// The bit buffer: 32 symbols of at most 1 + 32 (the run's zero and remainder)
+// + 64 bits (a Golomb-Rice code, escaped ones included) after up to 31 carried
+// over, with two words of slack for a code's 96-bit placement; also holds 1,023
+// bits kept and a chunk's 32 codes of 32 bits.
+constexpr int kEncBufWords = (31 + 32 * 97) / 32 + 3;
+
+struct EncShared {
+    int32_t sym[3][kEncRow * kEncChunk];      // chunk i % 3: the symbols
+    uint32_t st[2][kEncRow * kEncChunk];      // chunk i % 2: the state before each symbol
+    uint16_t mhigh[2][kEncRow * kEncChunk];   // ... and m >> 16 in a wide chunk
+    uint32_t wide[2];
+    uint32_t buf[32][kEncBufWords];           // the slices' bit buffers
+    uint32_t nbits[32];                       // bits in buf[f]: below 1024 between chunks
+    uint64_t nwords[32], cap[32];             // words out, words that fit
+    uint32_t* dst[32];
+    uint32_t end_kp[32], end_m[32];           // the state after the last symbol
+    uint8_t act[32], trail[32];               // has a slice; its last symbol was read in run mode and left u = 0
 };
 
-constexpr uint64_t kL = 4, kU0 = 3, kD0 = 1, kU1 = 2, kD1 = 1;
+__device__ __forceinline__ uint32_t shr_clamp(uint32_t v, uint32_t n) {  // v >> n, 0 for n >= 32
+    uint32_t d;
+    asm("shr.u32 %0, %1, %2;" : "=r"(d) : "r"(v), "r"(n));
+    return d;
+}
 
-constexpr int kEncRlgrBlock = 128;
-constexpr int kEncPf = 16;  // symbols per prefetch batch
-// The largest slices (first in `order`) are encoded kEncLongLanes to a warp
-// by the first CTAs of the launch, the rest kEncRestLanes to a warp: the
-// encoder's branches diverge between lanes, and a warp of 32 long slices
-// would take their divergent paths one after another.
-constexpr int kEncLongLanes = 2;
-constexpr int kEncLongCtas = 304;
-constexpr int kEncLongSlices = kEncLongCtas * (kEncRlgrBlock / 32) * kEncLongLanes;
-constexpr int kEncRestLanes = 32;
+// a symbol and the state it is coded in
+struct EncSymbol {
+    uint32_t uu, kr, k, m;
+    bool run, skip, full;  // skip: a zero inside a run; full: it completes 2^k of them
+    __device__ __forceinline__ EncSymbol(int32_t x, uint32_t st, uint32_t mhigh) {
+        const uint32_t u = ((uint32_t)x << 1) ^ (uint32_t)(x >> 31);  // Sign2Unsign
+        k = (st & 0xFFu) >> 2;
+        kr = (st >> 10) & 0x3Fu;
+        m = st >> 16 | mhigh << 16;
+        run = k != 0;
+        skip = run && u == 0;
+        full = ((m + 1) >> (k & 31)) != 0;
+        uu = u - (run && u != 0 ? 1u : 0u);
+    }
+    __device__ __forceinline__ uint32_t p() const { return shr_clamp(uu, kr); }
+};
 
-__global__ void __launch_bounds__(kEncRlgrBlock) k_rlgr_enc(const SliceWork* __restrict__ work,
-                                                           const int32_t* __restrict__ order, int nslices, int nlong,
-                                                           int long_ctas,
-                           const int32_t* __restrict__ sym, uint8_t* __restrict__ out, const uint64_t* __restrict__ out_off,
-                           const uint32_t* __restrict__ out_cap, uint32_t* __restrict__ out_len,
-                           int32_t* __restrict__ fstatus) {
-    __shared__ int32_t s_sym[kEncPf][kEncRlgrBlock];  // column threadIdx.x: this thread's batch
-    const int lane = threadIdx.x & 31;
-    int t;
-    if ((int)blockIdx.x < long_ctas) {
-        t = ((int)blockIdx.x * (kEncRlgrBlock / 32) + (int)(threadIdx.x >> 5)) * kEncLongLanes + lane;
-        if (lane >= kEncLongLanes || t >= nlong) return;
-    } else {
-        t = nlong + (((int)blockIdx.x - long_ctas) * (kEncRlgrBlock / 32) + (int)(threadIdx.x >> 5)) * kEncRestLanes + lane;
-        if (lane >= kEncRestLanes || t >= nslices) return;
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
     }
-    const int item = order[t];
-    const SliceWork& w = work[item];
-    if (fstatus[item] != PVVC_OK) {
-        out_len[w.orig] = 0;
-        return;
-    }
-    const uint32_t N = w.n;
-    const int32_t* s = sym + w.coef_off + w.coef_lane;
-    const size_t cs = w.coef_stride;
-    BitSink bw{reinterpret_cast<uint32_t*>(out + out_off[w.orig]), out_cap[w.orig]};
-    uint64_t u = 0, kP = 0, kRP = 2 * kL, m = 0, k = 0;
-    const uint64_t total = 3ull * N;
-    auto encode = [&](int64_t x) {
-        u = x < 0 ? ((uint64_t)(-x) << 1) - 1 : (uint64_t)x << 1;  // Sign2Unsign
-        k = kP / kL;
-        const uint64_t kR = kRP / kL;
-        if (k) {
-            if (u) {
-                --u;
-                bw.put(0, 1);
-                bw.put(m, (int)k);
-                bw.gr(u, (int)kR);
-                const uint64_t p = u >> kR;
-                kRP = p ? min(kRP + p - 1, 32 * kL) : (kRP < 2 ? 0 : kRP - 2);
-                kP = kP < kD1 ? 0 : kP - kD1;
-                m = 0;
-            } else if (++m == (1ull << k)) {
-                bw.put(1, 1);
-                kP += kU1;
-                m = 0;
-            }
-        } else {
-            bw.gr(u, (int)kR);
-            const uint64_t p = u >> kR;
-            kRP = p ? min(kRP + p - 1, 32 * kL) : (kRP < 2 ? 0 : kRP - 2);
-            kP = u ? (kP < kD0 ? 0 : kP - kD0) : kP + kU0;
-            m = 0;
+    return v;
+}
+
+// OR the low `len` (<= 64) bits of v into the MSB-first bit buffer at bit `at`
+__device__ __forceinline__ void put_bits(uint32_t* buf, uint32_t at, uint64_t v, uint32_t len) {
+    if (len == 0) return;
+    v <<= 64 - len;
+    const uint32_t w = at >> 5, s = at & 31;
+    const uint32_t hi = (uint32_t)(v >> 32), lo = (uint32_t)v;
+    const uint32_t a = hi >> s, b = __funnelshift_r(lo, hi, s), c = __funnelshift_r(0u, lo, s);
+    if (a) atomicOr(buf + w, a);
+    if (b) atomicOr(buf + w + 1, b);
+    if (c) atomicOr(buf + w + 2, c);
+}
+
+__global__ void __launch_bounds__(32 * kEncWarpsR) k_rlgr_enc(const SliceWork* __restrict__ work,
+                                                              const GroupDesc* __restrict__ groups,
+                                                              const int32_t* __restrict__ items,
+                                                              const int32_t* __restrict__ sym, uint8_t* __restrict__ out,
+                                                              const uint64_t* __restrict__ out_off,
+                                                              const uint32_t* __restrict__ out_cap,
+                                                              uint32_t* __restrict__ out_len, int32_t* __restrict__ fstatus) {
+    extern __shared__ __align__(16) unsigned char s_enc[];
+    EncShared& e = *reinterpret_cast<EncShared*>(s_enc);
+    __shared__ uint32_t s_n;
+    __shared__ uint64_t s_region;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const GroupDesc G = groups[blockIdx.x];
+    if (wid == 0) {
+        bool act = false;
+        uint32_t n = 0;
+        uint64_t region = 0;
+        if (lane < G.count) {
+            const int item = items[G.first + lane];
+            const SliceWork& w = work[item];
+            act = fstatus[item] == PVVC_OK;
+            e.dst[lane] = reinterpret_cast<uint32_t*>(out + out_off[w.orig]);
+            e.cap[lane] = out_cap[w.orig] / 4;
+            n = w.n;
+            region = w.coef_off;
+            if (!act) out_len[w.orig] = 0;
         }
+        e.act[lane] = act;
+        e.trail[lane] = 0;
+        e.nbits[lane] = 0;
+        e.nwords[lane] = 0;
+        // the good slices of a group have their slot's leaf count
+        const uint32_t bal = __ballot_sync(0xffffffffu, act);
+        if (bal) {
+            n = __shfl_sync(0xffffffffu, n, __ffs(bal) - 1);
+            region = __shfl_sync(0xffffffffu, region, __ffs(bal) - 1);
+        }
+        if (lane == 0) {
+            s_n = bal ? n : 0u;
+            s_region = region;
+        }
+    }
+    for (int i = tid; i < 32 * kEncBufWords; i += 32 * kEncWarpsR) e.buf[0][i] = 0;
+    __syncthreads();
+    const uint64_t total = 3ull * s_n;
+    const uint64_t nch = (total + kEncChunk - 1) / kEncChunk;
+    const int32_t* const src = sym + s_region;
+    auto fetch = [&](uint64_t c) {  // chunk c's symbols (position j of the planes: 32 lanes at j * 32)
+        if (c < nch) {
+            int32_t* const to = e.sym[c % 3];
+            for (uint32_t i = tid; i < 32 * kEncChunk; i += 32 * kEncWarpsR) {
+                const uint64_t j = c * kEncChunk + (i >> 5);
+                if (j < total)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(to + enc_at(i >> 5, i & 31))),
+                                 "l"(src + j * 32 + (i & 31))
+                                 : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    // The symbols of a slice sit coef_stride apart (frame-interleaved planes),
-    // one sector each: they are loaded kEncPf at a time into registers, the
-    // next batch in flight while this one is encoded from the thread's own
-    // shared-memory column, so the chain does not wait on every load.
-    int32_t nxt[kEncPf];
-#pragma unroll
-    for (int j = 0; j < kEncPf; ++j) nxt[j] = (uint64_t)j < total ? s[(uint64_t)j * cs] : 0;
-    for (uint64_t b0 = 0; b0 < total && !bw.overflow; b0 += kEncPf) {
-        uint32_t nz = 0;  // bit j: symbol b0 + j is nonzero
-#pragma unroll
-        for (int j = 0; j < kEncPf; ++j) {
-            s_sym[j][threadIdx.x] = nxt[j];
-            nz |= (uint32_t)(nxt[j] != 0) << j;
+    // the full words of slice f's buffer (n bits) out, the rest carried to its front
+    auto flush = [&](int f, uint32_t n) {
+        uint32_t* const buf = e.buf[f];
+        const uint32_t full = n >> 5;
+        const uint64_t nw = e.nwords[f], cap = e.cap[f];
+        __syncwarp();
+        const uint32_t carry = buf[full];
+        for (uint32_t i = lane; i < full; i += 32)
+            if (nw + i < cap) e.dst[f][nw + i] = __byte_perm(buf[i], 0, 0x0123);
+        __syncwarp();
+        for (uint32_t i = lane; i <= full; i += 32) buf[i] = i == 0 ? carry : 0u;
+        if (lane == 0) {
+            e.nwords[f] = nw + full;
+            e.nbits[f] = n & 31u;
         }
-        if (b0 + kEncPf < total) {
+        __syncwarp();
+    };
+    uint32_t kP = 0, kRP = 8, m = 0;  // warp 0, lane f: slice f's state
+    fetch(0);
+    for (uint64_t i = 0; i <= nch; ++i) {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();  // chunk i is in, the states of chunk i - 1 are written, chunk i - 2 is coded
+        fetch(i + 1);
+        if (wid == 0) {
+            if (i < nch) {
+                const int32_t* const S = e.sym[i % 3];
+                uint32_t* const T = e.st[i & 1];
+                uint16_t* const M = e.mhigh[i & 1];
+                const bool wide = __any_sync(0xffffffffu, kP >= kEncWideP);
+                if (lane == 0) e.wide[i & 1] = wide;
+                const uint32_t cnt = (uint32_t)min(total - i * kEncChunk, (uint64_t)kEncChunk);
+                auto step = [&](uint32_t j, int32_t x) {
+                    const uint32_t u = ((uint32_t)x << 1) ^ (uint32_t)(x >> 31);  // Sign2Unsign
+                    T[enc_at(j, lane)] = (m << 16) + (kRP << 8) + kP;
+                    const bool run = kP >= 4, zero = u == 0, skip = run && zero;
+                    // p = (u - run) >> kR, capped (any p above kMaxRP saturates kRP);
+                    // kRP + p - 1, or kRP - 2 for p = 0, without a predicate: this
+                    // chain is the longest
+                    const uint32_t p = min(shr_clamp(run ? max(u, 1u) - 1u : u, kRP >> 2), kMaxRP + 1);
+                    const bool full = ((m + 1) >> (kP >> 2)) != 0;  // the run reaches 2^k zeros
+                    const uint32_t rp = (uint32_t)max(min((int)(kRP + p + min(p, 1u)) - 2, (int)kMaxRP), 0);
+                    const uint32_t zp = run ? (full ? kP + kU1 : kP) : kP + kU0;
+                    kP = zero ? zp : max(kP, 1u) - 1u;
+                    kRP = skip ? kRP : rp;
+                    m = skip && !full ? m + 1 : 0u;
+                };
+                if (cnt == kEncChunk && !wide) {
+                    // the symbols eight at a time, ahead of their steps: the
+                    // compiler keeps loads behind the states' stores
+                    int32_t x[8];
 #pragma unroll
-            for (int j = 0; j < kEncPf; ++j) nxt[j] = b0 + kEncPf + j < total ? s[(b0 + kEncPf + j) * cs] : 0;
-        }
-        const int cnt = total - b0 < (uint64_t)kEncPf ? (int)(total - b0) : kEncPf;
-        int j = 0;
-        while (j < cnt) {
-            const int32_t x = s_sym[j][threadIdx.x];
-            if (x != 0 || kP < kL) {
-                encode(x);
-                ++j;
-                continue;
-            }
-            // Zeros in run mode, taken together: each symbol would add one to
-            // m and, when m reaches 2^k, write a 1 and raise kP by kU1 (k only
-            // grows, so the run stays in run mode).  `k` ends as the value the
-            // last zero saw, as the trailing-run test after the loop expects.
-            const uint32_t rest = nz >> j;
-            int z = rest ? __ffs(rest) - 1 : cnt - j;
-            if (z > cnt - j) z = cnt - j;
-            j += z;
-            uint64_t left = (uint64_t)z;
-            while (left) {
-                k = kP / kL;
-                const uint64_t need = (1ull << k) - m;
-                if (left >= need) {
-                    left -= need;
-                    bw.put(1, 1);
-                    kP += kU1;
-                    m = 0;
+                    for (uint32_t j = 0; j < 8; ++j) x[j] = S[enc_at(j, lane)];
+#pragma unroll
+                    for (uint32_t j0 = 0; j0 < kEncChunk; j0 += 8) {
+                        int32_t y[8];
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j) y[j] = j0 + 8 < kEncChunk ? S[enc_at(j0 + 8 + j, lane)] : 0;
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j) step(j0 + j, x[j]);
+#pragma unroll
+                        for (uint32_t j = 0; j < 8; ++j) x[j] = y[j];
+                    }
                 } else {
-                    m += left;
-                    left = 0;
+                    for (uint32_t j = 0; j < cnt; ++j) {
+                        M[enc_at(j, lane)] = (uint16_t)(m >> 16);
+                        step(j, S[enc_at(j, lane)]);
+                    }
+                }
+                if (i + 1 == nch) {
+                    e.end_kp[lane] = kP;
+                    e.end_m[lane] = m;
                 }
             }
-            u = 0;
+        } else if (i > 0 && (wid & 3) != 0) {  // (warps 4, 8, .. would share warp 0's scheduler)
+            const uint64_t c = i - 1;
+            const uint32_t cnt = (uint32_t)min(total - c * kEncChunk, (uint64_t)kEncChunk);
+            const int32_t* const S = e.sym[c % 3];
+            const uint32_t* const T = e.st[c & 1];
+            const uint16_t* const M = e.mhigh[c & 1];
+            const bool wide_m = e.wide[c & 1] != 0;
+            for (int f = wid - 1 - (wid >> 2); f < G.count; f += kEncCoders) {
+                if (!e.act[f]) continue;
+                uint32_t code = 0, len = 0;
+                bool wide = false;
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    const uint32_t j = 2 * lane + h, at = enc_at(j, f);
+                    if (j >= cnt) continue;
+                    const EncSymbol y(S[at], T[at], wide_m ? M[at] : 0u);
+                    const uint32_t p = y.p();
+                    uint32_t n = p + 1 + y.kr + (y.run ? 1 + y.k : 0u);
+                    uint32_t v = (((2u << (p & 31)) - 2u) << (y.kr & 31)) | (y.uu & ((1u << (y.kr & 31)) - 1u));
+                    v |= y.run ? __funnelshift_lc(0u, y.m, p + 1 + y.kr) : 0u;
+                    if (y.skip) n = v = y.full ? 1u : 0u;  // a completed run: a 1
+                    wide |= n > 32 || p >= 32 || len + n > 32;
+                    code = __funnelshift_lc(0u, code, n) | v;
+                    len += n;
+                    if (c + 1 == nch && j == cnt - 1) e.trail[f] = y.run && y.uu == 0;
+                }
+                if (__any_sync(0xffffffffu, wide)) {
+                    flush(f, e.nbits[f]);
+                    for (uint32_t h = 0; h < kEncChunk; h += 32) {
+                        uint64_t head = 0, body = 0;
+                        uint32_t hlen = 0, blen = 0;
+                        if (h + lane < cnt) {
+                            const uint32_t at = enc_at(h + lane, f);
+                            const EncSymbol y(S[at], T[at], wide_m ? M[at] : 0u);
+                            const uint32_t p = y.p();
+                            if (y.skip) {
+                                body = blen = y.full ? 1u : 0u;
+                            } else {
+                                if (y.run) {  // the run's end: a zero and its remainder
+                                    head = y.m;
+                                    hlen = 1 + y.k;
+                                }
+                                if (p < 32) {  // GRWrite: p ones, a zero, kR bits
+                                    body = (((1ull << (p + 1)) - 2) << y.kr) | (y.uu & (uint32_t)((1ull << y.kr) - 1));
+                                    blen = p + 1 + y.kr;
+                                } else {
+                                    body = 0xFFFFFFFF00000000ull | y.uu;
+                                    blen = 64;
+                                }
+                            }
+                        }
+                        const uint32_t n = hlen + blen;
+                        const uint32_t end = warp_incl_scan(n, lane), bits = __shfl_sync(0xffffffffu, end, 31);
+                        if (bits == 0) continue;
+                        const uint32_t nb = e.nbits[f], at = nb + end - n;
+                        put_bits(e.buf[f], at, head, hlen);
+                        put_bits(e.buf[f], at + hlen, body, blen);
+                        flush(f, nb + bits);
+                    }
+                    continue;
+                }
+                const uint32_t end = warp_incl_scan(len, lane), bits = __shfl_sync(0xffffffffu, end, 31);
+                if (bits == 0) continue;
+                const uint32_t nb = e.nbits[f];
+                if (len) {
+                    const uint32_t at = nb + end - len, w = at >> 5, sh = at & 31, v = code << (32 - len);
+                    atomicOr(&e.buf[f][w], v >> sh);
+                    if (sh + len > 32) atomicOr(&e.buf[f][w + 1], __funnelshift_r(0u, v, sh));
+                }
+                // out once a line's worth of words is full
+                if (nb + bits >= 1024) {
+                    flush(f, nb + bits);
+                } else {
+                    __syncwarp();
+                    if (lane == 0) e.nbits[f] = nb + bits;
+                    __syncwarp();
+                }
+            }
         }
     }
-    if (total > 0 && k && !u) {  // trailing run (entropy_codec.cc:144-147)
-        bw.put(0, 1);
-        bw.put(m, (int)(kP / kL));
+    __syncthreads();
+    for (int f = wid; f < G.count; f += kEncWarpsR) {
+        if (!e.act[f]) continue;
+        flush(f, e.nbits[f]);
+        if (e.trail[f]) {  // trailing run (entropy_codec.cc:144-147)
+            const uint32_t n = 1 + (e.end_kp[f] >> 2), nb = e.nbits[f];
+            if (lane == 0) put_bits(e.buf[f], nb, e.end_m[f], n);
+            flush(f, nb + n);
+        }
+        if (lane == 0) {  // zero bits up to the byte boundary
+            const uint32_t nb = e.nbits[f];
+            const uint64_t nw = e.nwords[f], cap = e.cap[f], nbytes = nw * 4 + ((nb + 7) >> 3);
+            const int item = items[G.first + f];
+            const SliceWork& w = work[item];
+            if (nb && nw < cap) e.dst[f][nw] = __byte_perm(e.buf[f][0], 0, 0x0123);
+            out_len[w.orig] = nbytes > cap * 4 ? 0u : (uint32_t)nbytes;
+            if (nbytes > cap * 4) fstatus[item] = PVVC_ERR_CAPACITY;
+        }
     }
-    bw.finish();
-    out_len[w.orig] = bw.overflow ? 0 : bw.nbytes;
-    if (bw.overflow) fstatus[item] = PVVC_ERR_CAPACITY;
 }
 
 __global__ void k_status_out(const SliceWork* __restrict__ work, int n, const int32_t* __restrict__ fstatus,
@@ -421,20 +576,17 @@ extern "C" int pvvc_encode_colors(pvvc_encoder* enc, const pvvc_batch_desc* desc
         cudaMemcpyAsync(enc->cap.p, enc->h_cap.p, 4ull * n, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaMemsetAsync(cnt, 0, sizeof(int), s) != cudaSuccess)
         return PVVC_ERR_CUDA;
-    if (launch_tree(dw, p.nintra, payload, st->v, ts, s) != cudaSuccess) return PVVC_ERR_CUDA;
+    if (launch_tree(dw, p.nintra, payload, st->v, ts, s) != cudaSuccess ||
+        cudaFuncSetAttribute(k_rlgr_enc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EncShared)) != cudaSuccess)
+        return PVVC_ERR_CUDA;
     const int ng = p.ngroups_a + p.ngroups_b;
     const int grid = std::min(ng, std::max(p.grp_ctas, 1));
     k_fwd_raht<<<grid, 32 * kEncWarps, 0, s>>>(dw, static_cast<const GroupDesc*>(p.d_groups.p), ng,
                                                static_cast<const int32_t*>(p.d_idx.p), st->v, leaf_yuv, sym, ts, fs, scr,
                                                p.grp_floats, cnt);
-    const int nlong = n < kEncLongSlices ? n : kEncLongSlices;
-    const int per_long_cta = (kEncRlgrBlock / 32) * kEncLongLanes;
-    const int long_ctas = (nlong + per_long_cta - 1) / per_long_cta;
-    const int per_rest_cta = (kEncRlgrBlock / 32) * kEncRestLanes;
-    k_rlgr_enc<<<long_ctas + (n - nlong + per_rest_cta - 1) / per_rest_cta, kEncRlgrBlock, 0, s>>>(
-        dw, static_cast<const int32_t*>(p.d_order.p), n, nlong, long_ctas, sym, out,
-                                                static_cast<const uint64_t*>(enc->off.p),
-                                                static_cast<const uint32_t*>(enc->cap.p), out_len, fs);
+    k_rlgr_enc<<<ng, 32 * kEncWarpsR, sizeof(EncShared), s>>>(
+        dw, static_cast<const GroupDesc*>(p.d_groups.p), static_cast<const int32_t*>(p.d_idx.p), sym, out,
+        static_cast<const uint64_t*>(enc->off.p), static_cast<const uint32_t*>(enc->cap.p), out_len, fs);
     k_status_out<<<(n + 255) / 256, 256, 0, s>>>(dw, n, fs, status);
     if (cudaGetLastError() != cudaSuccess) return PVVC_ERR_CUDA;
     // the host arrays above are reused by the next call: finish this one

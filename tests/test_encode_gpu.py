@@ -138,3 +138,34 @@ def test_gpu_encoder_reports_capacity(pvvc_lib, torch):
                torch.cuda.current_stream().cuda_stream)
     torch.cuda.synchronize()
     assert (st.cpu().numpy() == 11).all() and (olen.cpu().numpy() == 0).all()
+
+
+@pytest.mark.parametrize("side,nframes", [(51, 2), (3, 33), (4, 1)])
+def test_gpu_encoder_runs_and_chunk_edges(pvvc_lib, torch, side, nframes):
+    """Constant colours on a full cube: runs whose remainder passes 16 bits
+    (51^3 voxels: 17-bit remainders in the V plane); more frames than lanes,
+    and slices of 81 and 192 symbols (a partial and three full chunks of 64).
+    The second patch's large alternating colours need codes beyond 32 bits."""
+    rng = np.random.default_rng(side)
+    cube = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij"), -1).reshape(-1, 3).astype(np.float32)
+    flat = np.full((nframes, cube.shape[0], 3), 40.0, np.float32)
+    small = rng.integers(0, 6, (120, 3)).astype(np.float32)
+    loud = (rng.integers(0, 2, (nframes, 120, 3)) * 60000.0 - 30000.0).astype(np.float32)
+    qps = [1 + f % 4 for f in range(nframes)]
+    patches = [(cube, flat), (small, loud)]
+    frames, batch, leaf_yuv, cpu = _gop(pvvc_lib, patches, qps)
+    dec = pvvc_lib.Decoder(nslots=2, max_leaves=max(cube.shape[0], 8192))
+    enc = pvvc_lib.Encoder()
+    cap = ((16 * batch.size.astype(np.uint64) + 64 + 3) // 4 * 4).astype(np.uint32)
+    off = np.concatenate([[0], np.cumsum(cap.astype(np.uint64))[:-1]]).astype(np.uint64)
+    pay, ly = _dev(torch, batch.payload), _dev(torch, leaf_yuv)
+    out = torch.zeros(int(cap.astype(np.uint64).sum()) + 16, dtype=torch.uint8, device="cuda")
+    olen = torch.zeros(batch.nslices, dtype=torch.int32, device="cuda")
+    st = torch.full((batch.nslices,), -1, dtype=torch.int32, device="cuda")
+    enc.encode(batch, dec, pay.data_ptr(), ly.data_ptr(), out.data_ptr(), off, cap, olen.data_ptr(), st.data_ptr(),
+               torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert (st.cpu().numpy() == 0).all()
+    o, lens = out.cpu().numpy(), olen.cpu().numpy()
+    for k in range(batch.nslices):
+        assert o[int(off[k]):int(off[k]) + int(lens[k])].tobytes() == cpu[k % 2][k // 2], k
