@@ -12,11 +12,13 @@
 //            histogram + block scan), written to the workspace as float4
 //            (x, y, z, index of the point in its pair).
 //   k_icp    one CTA per pair, all iterations: each thread transforms its
-//            source points, finds the exact nearest target point by rings of
-//            grid cells (FP32), and accumulates the correspondence sums with
-//            Kahan-compensated FP32 additions; the block reduces them in FP64
-//            and one thread solves the 3x3 Kabsch problem by a Jacobi SVD in
-//            FP64 and applies the convergence tests of the PCL criteria.
+//            source points, finds the exact nearest target point among the
+//            grid cells around the last iteration's (FP32), and accumulates
+//            the correspondence sums with Kahan-compensated FP32 additions;
+//            the block reduces them in FP64 and one warp solves the 3x3
+//            Kabsch problem in FP64 (polar decomposition; Jacobi SVD for
+//            near-singular ones) and applies the convergence tests of the
+//            PCL criteria.
 //   k_nn_mean  mean squared NN distance of (transformed) query points to a
 //            gridded cloud, per pair.
 //   k_knn_color  colour interpolation of the GoP encoder (k nearest source
@@ -24,10 +26,12 @@
 //            k_knn_sub turns later frames into residuals against frame 0.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 #include <mutex>
 
+#include "decode_internal.h"
 #include "pvvc_gb300.h"
 
 namespace pvvc {
@@ -60,7 +64,7 @@ struct GridHdr {  // per pair
     float lo[3];
     float h;
     int dim[3];
-    int pad;
+    float eps;  // bounds how far rounding can put a point outside its cell's box
 };
 
 // ---------------------------------------------------------------------------
@@ -158,7 +162,8 @@ __global__ void __launch_bounds__(T) k_grid(const float* __restrict__ pts, const
         s_box[3] = g.h;
         s_box[4] = __int_as_float(g.dim[0]);
         s_box[5] = __int_as_float(g.dim[1] * 1024 + g.dim[2]);
-        g.pad = 0;
+        g.eps = 0.f;
+        for (int k = 0; k < 3; ++k) g.eps = fmaxf(g.eps, 1e-6f * (fabsf(g.lo[k]) + e[k]));
         hdr[pair] = g;
     }
     __syncthreads();
@@ -213,71 +218,99 @@ __global__ void __launch_bounds__(T) k_grid(const float* __restrict__ pts, const
     }
 }
 
-// exact nearest neighbour: squared distance (and the point) of the closest
-// gridded point to q, searching rings of cells around q's cell clamped into
-// the grid; a point in ring r lies at least (r-1)*h from q.  Among points at
-// the same distance the one first in the input wins, so the answer does not
-// depend on the grid's cell size or on the order the cells are visited in.
-__device__ __forceinline__ float grid_nn(const GridHdr& g, const int* __restrict__ cs, const float4* __restrict__ sp, uint32_t base,
-                                         float qx, float qy, float qz, float* nx, float* ny, float* nz) {
-    const int cx = min(max((int)floorf((qx - g.lo[0]) / g.h), 0), g.dim[0] - 1);
-    const int cy = min(max((int)floorf((qy - g.lo[1]) / g.h), 0), g.dim[1] - 1);
-    const int cz = min(max((int)floorf((qz - g.lo[2]) / g.h), 0), g.dim[2] - 1);
-    float best = FLT_MAX;
-    float bx = 0.f, by = 0.f, bz = 0.f;
+// Exact nearest neighbour of q among the gridded points sp[0 ..): the one first
+// in the input among points at the same distance, so the answer does not depend
+// on the grid's cell size or on the order the cells are visited in.
+//
+// The search starts from a point known to be near (`start`, an index into sp;
+// -1: none, then rings of cells around q's cell until one holds a point) and
+// visits the rows of cells that meet the ball around q through the best point so
+// far; the cells of a row are neighbours in sp, so a row is one run of points.
+//
+// A cell's box is widened by eps (rounding of the cell assignment), the last
+// cell of an axis is open upwards (it also holds what a clamped axis leaves
+// over), and squared bounds keep a margin of 1e-4, so no point that could win
+// is skipped.
+struct NearPoint {
+    float d;       // squared distance; FLT_MAX: none
+    int j;         // into sp; -1: none
+};
+__device__ __forceinline__ float sqrt_fast(float x) {
+    float y;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float dist2(const float4& p, float qx, float qy, float qz) {
+    const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
+    return dx * dx + dy * dy + dz * dz;
+}
+__device__ __forceinline__ NearPoint grid_nn(const GridHdr& g, const int* __restrict__ cs, const float4* __restrict__ sp,
+                                             float qx, float qy, float qz, int start) {
+    NearPoint r{FLT_MAX, -1};
     int bi = 0x7fffffff;
-    const int maxr = max(g.dim[0], max(g.dim[1], g.dim[2]));
-    for (int r = 0; r <= maxr; ++r) {
-        if (r > 0 && best < FLT_MAX) {
-            const float lb = (float)(r - 1) * g.h;
-            if (lb * lb * 0.999f > best) break;
+    auto visit = [&](int k) {
+        const float4 p = __ldg(sp + k);
+        const float d = dist2(p, qx, qy, qz);
+        const int pi = __float_as_int(p.w);
+        if (d < r.d || (d == r.d && pi < bi)) {
+            r.d = d;
+            r.j = k;
+            bi = pi;
         }
-        for (int z = max(cz - r, 0); z <= min(cz + r, g.dim[2] - 1); ++z) {
-            const bool zr = (z == cz - r) || (z == cz + r);
-            // squared distance from q to the cell's box along an axis
-            auto gap2 = [&](int c, float q, float lo) {
-                const float a = lo + (float)c * g.h, b = a + g.h;
-                const float d = q < a ? a - q : (q > b ? q - b : 0.f);
-                return d * d;
-            };
-            const float dz2 = gap2(z, qz, g.lo[2]);
-            if (dz2 * 0.999f > best) continue;
-            for (int y = max(cy - r, 0); y <= min(cy + r, g.dim[1] - 1); ++y) {
-                const float dyz2 = dz2 + gap2(y, qy, g.lo[1]);
-                if (dyz2 * 0.999f > best) continue;
-                const bool yr = zr || (y == cy - r) || (y == cy + r);
-                // on interior rows only the two x faces belong to the ring
-                int x = max(cx - r, 0);
-                const int xe = min(cx + r, g.dim[0] - 1);
-                const int step = yr ? 1 : max(2 * r, 1);
-                if (!yr && x != cx - r) x = (cx + r <= xe) ? cx + r : xe + 1;
-                for (; x <= xe; x += step) {
-                    // a cell farther than the best so far cannot hold a strictly
-                    // closer point (0.999: margin for the rounding of the bound)
-                    if ((dyz2 + gap2(x, qx, g.lo[0])) * 0.999f > best) continue;
-                    const int c = (z * g.dim[1] + y) * g.dim[0] + x;
-                    const int e = __ldg(cs + c + 1);
-                    for (int k = __ldg(cs + c); k < e; ++k) {
-                        const float4 p = __ldg(sp + base + k);
-                        const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
-                        const float d = dx * dx + dy * dy + dz * dz;
-                        const int pi = __float_as_int(p.w);
-                        if (d < best || (d == best && pi < bi)) {
-                            best = d;
-                            bi = pi;
-                            bx = p.x;
-                            by = p.y;
-                            bz = p.z;
-                        }
+    };
+    const float inv = 1.0f / g.h;
+    auto cell = [&](float v, int k) { return min(max((int)floorf((v - g.lo[k]) * inv), 0), g.dim[k] - 1); };
+    if (start >= 0) visit(start);
+    if (r.j < 0) {
+        const int cx = cell(qx, 0), cy = cell(qy, 1), cz = cell(qz, 2);
+        const int maxr = max(g.dim[0], max(g.dim[1], g.dim[2]));
+        for (int t = 0; t <= maxr && r.j < 0; ++t)
+            for (int z = max(cz - t, 0); z <= min(cz + t, g.dim[2] - 1); ++z)
+                for (int y = max(cy - t, 0); y <= min(cy + t, g.dim[1] - 1); ++y) {
+                    const int row = (z * g.dim[1] + y) * g.dim[0];
+                    // on interior rows only the two x faces belong to the ring
+                    const bool face = abs(z - cz) == t || abs(y - cy) == t;
+                    const int x0 = max(cx - t, 0), x1 = min(cx + t, g.dim[0] - 1);
+                    if (face) {
+                        for (int k = __ldg(cs + row + x0), e = __ldg(cs + row + x1 + 1); k < e; ++k) visit(k);
+                    } else {
+                        if (cx - t >= 0)
+                            for (int k = __ldg(cs + row + x0), e = __ldg(cs + row + x0 + 1); k < e; ++k) visit(k);
+                        if (cx + t < g.dim[0])
+                            for (int k = __ldg(cs + row + x1), e = __ldg(cs + row + x1 + 1); k < e; ++k) visit(k);
                     }
                 }
+        if (r.j < 0) return r;
+    }
+    // the ball to the best point
+    float at = r.d, rad = sqrt_fast(r.d) * 1.0001f + g.eps;
+    const float rad0 = rad;
+    auto gap = [&](int c, float q, int k) {
+        const float a = g.lo[k] + (float)c * g.h;
+        const float d = q < a ? a - q : (q > a + g.h && c < g.dim[k] - 1 ? q - (a + g.h) : 0.f);
+        return fmaxf(d - g.eps, 0.f);
+    };
+    const float pad = 0.001f * g.h + g.eps;  // of the cell indices' rounding
+    const int z1 = cell(qz + rad0 + pad, 2), y0 = cell(qy - rad0 - pad, 1), y1 = cell(qy + rad0 + pad, 1);
+    for (int z = cell(qz - rad0 - pad, 2); z <= z1; ++z) {
+        const float gz = gap(z, qz, 2), gz2 = gz * gz;
+        if (gz2 * 0.9999f > rad * rad) continue;
+        for (int y = y0; y <= y1; ++y) {
+            const float gy = gap(y, qy, 1), g2 = gz2 + gy * gy;
+            const float left = rad * rad - g2 * 0.9999f;
+            if (left < 0.f) continue;
+            const float rx = sqrt_fast(left) * 1.0001f + pad;
+            const int row = (z * g.dim[1] + y) * g.dim[0];
+            const int e = __ldg(cs + row + cell(qx + rx, 0) + 1);
+            for (int k = __ldg(cs + row + cell(qx - rx, 0)); k < e; ++k)
+                visit(k);
+            if (r.d != at) {  // a closer point: the ball shrinks
+                at = r.d;
+                rad = sqrt_fast(r.d) * 1.0001f + g.eps;
             }
         }
     }
-    *nx = bx;
-    *ny = by;
-    *nz = bz;
-    return best;
+    return r;
 }
 
 // ---- FP64 3x3 Kabsch (one-sided Jacobi SVD) ---------------------------------
@@ -325,14 +358,10 @@ __device__ void svd3(const double* A, double* U, double* S, double* V) {
     }
 }
 
-__device__ void kabsch(double n, const double* sp, const double* sq, const double* spq, double* R, double* t) {
-    double cp[3], cq[3], H[9], U[9], S[3], V[9];
-    for (int a = 0; a < 3; ++a) {
-        cp[a] = sp[a] / n;
-        cq[a] = sq[a] / n;
-    }
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) H[3 * i + j] = spq[3 * i + j] - n * cp[i] * cq[j];
+// The rotation of Kabsch's problem by Jacobi SVD: R = V U^T, the direction of
+// the smallest singular value flipped when that is a reflection.
+__device__ __noinline__ void kabsch_svd(const double* H, double* R) {
+    double U[9], S[3], V[9];
     svd3(H, U, S, V);
     auto vut = [&]() {
         for (int i = 0; i < 3; ++i)
@@ -347,7 +376,64 @@ __device__ void kabsch(double n, const double* sp, const double* sq, const doubl
         for (int i = 0; i < 3; ++i) V[3 * i + k] = -V[3 * i + k];
         vut();
     }
-    for (int i = 0; i < 3; ++i) t[i] = cq[i] - (R[3 * i] * cp[0] + R[3 * i + 1] * cp[1] + R[3 * i + 2] * cp[2]);
+}
+
+// The same rotation as the orthogonal polar factor of H^T, by Higham's scaled
+// Newton iteration X <- (g X + X^-T / g) / 2 (N. J. Higham, "Computing the polar
+// decomposition -- with applications", 1986), one warp: lane 3 i + j holds
+// element (i, j).  It needs a division and a handful of dependent FP64
+// operations a round (63 cycles each on this GPU, a division 590, a square root
+// 630) where a Jacobi rotation needs three divisions and three square roots, and
+// its sums over lanes instead of one after another: with warp_sums17 an ICP
+// iteration of 16 points takes 18 us, 60 with the SVD and plain butterflies.
+// True (in every lane) when it settled on a rotation: H with a positive
+// determinant, not near-singular (the smallest singular value above some 1e-5 of
+// the others); otherwise the caller takes kabsch_svd.
+__device__ __forceinline__ bool polar3(double h, int lane, double* r) {
+    const unsigned full = 0xffffffffu;
+    const int l = lane < 9 ? lane : 0, i = l / 3, j = l % 3;
+    const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+    // X = H^T, scaled by the largest entry
+    double x = __shfl_sync(full, h, 3 * j + i);
+    float big = lane < 9 ? fabsf((float)x) : 0.f;
+    for (int o = 8; o; o >>= 1) big = fmaxf(big, __shfl_xor_sync(full, big, o));
+    big = __shfl_sync(full, big, 0);
+    if (!(big > 1e-30f && big < 1e30f)) return false;
+    x *= (double)__frcp_rn(big);
+    float prev = FLT_MAX;
+    for (int round = 0; round < 24; ++round) {
+        // cofactors of X: X^-T = cof(X) / det(X)
+        const double c = __shfl_sync(full, x, 3 * i1 + j1) * __shfl_sync(full, x, 3 * i2 + j2) -
+                         __shfl_sync(full, x, 3 * i1 + j2) * __shfl_sync(full, x, 3 * i2 + j1);
+        const double xc = x * c;
+        const double det = (__shfl_sync(full, xc, 0) + __shfl_sync(full, xc, 1)) + __shfl_sync(full, xc, 2);
+        // scale: g^2 = ||X^-1|| / ||X|| (Frobenius), in float -- any g > 0 is a
+        // valid step, 1 once X is nearly orthogonal
+        float nx = lane < 9 ? (float)x * (float)x : 0.f, nc = lane < 9 ? (float)c * (float)c : 0.f;
+        for (int o = 8; o; o >>= 1) {
+            nx += __shfl_xor_sync(full, nx, o);
+            nc += __shfl_xor_sync(full, nc, o);
+        }
+        nx = __shfl_sync(full, nx, 0);
+        nc = __shfl_sync(full, nc, 0);
+        const float fd = (float)det;
+        if (!(fd > 1e-5f * nx * sqrtf(nx))) return false;
+        float g = 1.f;
+        if (prev > 1e-2f) g = sqrtf(sqrtf(nc / nx) / fd);
+        const double y = 0.5 * ((double)g * x + c / (det * (double)g));
+        float ch = lane < 9 ? fabsf((float)(y - x)) : 0.f;
+        for (int o = 8; o; o >>= 1) ch = fmaxf(ch, __shfl_xor_sync(full, ch, o));
+        ch = __shfl_sync(full, ch, 0);
+        x = y;
+        // quadratic convergence: a change below 1e-8 leaves an error below 1e-15
+        if (g == 1.f && ch < 1e-8f) {
+            *r = x;
+            return true;
+        }
+        if (!(ch < 1e30f)) return false;
+        prev = ch;
+    }
+    return false;
 }
 
 // Kahan-compensated FP32 accumulator
@@ -365,18 +451,62 @@ struct KSum {
 constexpr int kIcpThreads = 256;
 constexpr int kNSum = 17;  // count, sum p (3), sum q (3), sum p q^T (9), sum d^2
 
-__global__ void __launch_bounds__(kIcpThreads) k_icp(const float* __restrict__ src, const uint32_t* __restrict__ soff,
+// Sums v[0 .. 16] over a warp: at each of the five exchanges a lane keeps half
+// of its values and adds its partner's, 20 additions instead of 85.  Each sum
+// is the one a butterfly over the lanes (16, 8, 4, 2, 1) gives, bit for bit.
+// On return the lane holds sum number `*which` (-1: none).
+__device__ __forceinline__ double warp_sums17(double (&v)[kNSum], int lane, int* which) {
+    int base = 0, n = kNSum;
+#pragma unroll
+    for (int o = 16, w = kNSum; o; o >>= 1) {
+        const int lo = (w + 1) / 2;  // w: the values a lane may hold here
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < lo; ++i) {
+            const double a = v[i], b = lo + i < w ? v[lo + i] : 0.0;
+            const double got = __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+            v[i] = (up ? b : a) + got;
+        }
+        // (a lane's own count may be below w: its last value is then padding)
+        base += up ? lo : 0;
+        n = up ? n - lo : min(n, lo);
+        w = lo;
+    }
+    *which = n >= 1 ? base : -1;
+    return v[0];
+}
+
+// k_icp.  KEEP: `near_j` holds every source point's nearest target point, where
+// the next iteration's search starts: the ball to search is known at once, about
+// as large as the answer's.  The neighbours are exact in every iteration, so the
+// sums, the transforms and the iteration counts do not depend on it.  Without
+// KEEP (the entry point without scratch for the source) every search looks for
+// a first point itself.
+//
+// T threads search, each sum runs over kIcpThreads of them in a fixed order, so T
+// changes no result.  What bounds the kernel is the latency of the searches'
+// dependent loads and of the FP64 solve, one pair after another on an SM: few
+// pairs take CTAs of 1024 threads (472 pairs of 1,680 points, 49 iterations on
+// average: 12.2 ms; 512 threads 12.4, 256 threads 16.3), pairs enough to fill the
+// chip several times over take smaller ones, so that one pair's solve overlaps
+// others' searches (1,000 pairs: 16.9 ms with 512, 18.9 with 1024, 19.2 with
+// 256; 2,048: 27.6 with 256, 28.5, 34.3).  It was 39.7 ms (472 pairs), 40.7
+// (1,000) and 69.0 (2,048) with rings of cells searched from nothing.  Finer grids
+// held as bits (one row a word, or bricks of 4 x 4 x 4 under a level of blocks)
+// tested a third of the points but spent more instructions a cell: 22 to 39 ms.
+template <bool KEEP, int T>
+__global__ void __launch_bounds__(T, 1024 / T) k_icp(const float* __restrict__ src, const uint32_t* __restrict__ soff,
                                                      const uint32_t* __restrict__ toff, const GridHdr* __restrict__ hdr,
                                                      const int* __restrict__ cstart, const float4* __restrict__ tsorted,
-                                                     int kmul, const float* __restrict__ init, pvvc_icp_params prm,
+                                                     const float* __restrict__ init, pvvc_icp_params prm,
                                                      float* __restrict__ T_out, float* __restrict__ mse_out,
                                                      int32_t* __restrict__ iters_out, uint8_t* __restrict__ conv_out,
-                                                     uint32_t cap = 0xFFFFFFFFu) {
+                                                     uint32_t cap, int* near_j, uint32_t src_cap) {
     __shared__ double s_part[kIcpThreads / 32][kNSum];
     __shared__ double s_T[16];
+    __shared__ double s_H[9], s_R[9];
     __shared__ float s_Tf[12];
     __shared__ int s_done;
-    __shared__ double s_prev;
     const int pair = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const uint32_t a = soff[pair], b = soff[pair + 1];
     const uint32_t tb = toff[pair];
@@ -390,110 +520,147 @@ __global__ void __launch_bounds__(kIcpThreads) k_icp(const float* __restrict__ s
         return;
     }
     const GridHdr g = hdr[pair];
-    const int* cs = cstart + cell_base(kmul, tb, pair);
+    const int* const cs = cstart + cell_base(kIcpCellMul, tb, pair);
+    const float4* const sp = tsorted + tb;
     const bool empty_t = toff[pair + 1] == tb;
-    if (tid == 0) {
-        for (int i = 0; i < 16; ++i) s_T[i] = init ? (double)init[pair * 16 + i] : ((i % 5 == 0) ? 1.0 : 0.0);
-        s_done = 0;
-        s_prev = DBL_MAX;
-    }
+    // the scratch holds src_cap source points: a pair beyond it is searched afresh
+    const bool keep = KEEP && b <= src_cap;
+    if (tid < 16) s_T[tid] = init ? (double)init[pair * 16 + tid] : ((tid % 5 == 0) ? 1.0 : 0.0);
+    if (tid == 0) s_done = 0;
     __syncthreads();
     const double corr2 = (double)prm.max_corr_dist * (double)prm.max_corr_dist;
-    int it = 0, conv = 0;
+    // d > corr2 in double, decided in float: the largest float not above corr2
+    const float corr2f = __double2float_rd(corr2);
+    bool first = true;
+    auto moved = [&](uint32_t i, float& qx, float& qy, float& qz) {
+        const float x = __ldg(src + 3ull * i), y = __ldg(src + 3ull * i + 1), z = __ldg(src + 3ull * i + 2);
+        qx = s_Tf[0] * x + s_Tf[1] * y + s_Tf[2] * z + s_Tf[3];
+        qy = s_Tf[4] * x + s_Tf[5] * y + s_Tf[6] * z + s_Tf[7];
+        qz = s_Tf[8] * x + s_Tf[9] * y + s_Tf[10] * z + s_Tf[11];
+    };
+    // every source point's nearest target point under s_Tf
+    auto search = [&]() {
+        if (!keep || empty_t) return;
+        for (uint32_t i = a + tid; i < b; i += T) {
+            float qx, qy, qz;
+            moved(i, qx, qy, qz);
+            near_j[i] = grid_nn(g, cs, sp, qx, qy, qz, first ? -1 : near_j[i]).j;
+        }
+        if (T > kIcpThreads) __syncthreads();  // (else a thread sums the points it searched)
+    };
+    // source point i's nearest target point, and its squared distance
+    auto nearest = [&](uint32_t i, float qx, float qy, float qz, float4& m) -> float {
+        const int j = keep ? near_j[i] : grid_nn(g, cs, sp, qx, qy, qz, -1).j;
+        m = j >= 0 ? __ldg(sp + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+        return j >= 0 ? dist2(m, qx, qy, qz) : FLT_MAX;
+    };
+    int it = 0, conv = 0;       // warp 0
+    double prev_mse = DBL_MAX;  // warp 0
     while (true) {
         if (tid < 12) s_Tf[tid] = (float)s_T[tid];
         __syncthreads();
-        KSum acc[kNSum];
-        for (uint32_t i = a + tid; i < b && !empty_t; i += kIcpThreads) {
-            const float x = __ldg(src + 3ull * i), y = __ldg(src + 3ull * i + 1), z = __ldg(src + 3ull * i + 2);
-            const float qx = s_Tf[0] * x + s_Tf[1] * y + s_Tf[2] * z + s_Tf[3];
-            const float qy = s_Tf[4] * x + s_Tf[5] * y + s_Tf[6] * z + s_Tf[7];
-            const float qz = s_Tf[8] * x + s_Tf[9] * y + s_Tf[10] * z + s_Tf[11];
-            float mx, my, mz;
-            const float d = grid_nn(g, cs, tsorted, tb, qx, qy, qz, &mx, &my, &mz);
-            if ((double)d > corr2) continue;
-            acc[0].add(1.f);
-            acc[1].add(qx);
-            acc[2].add(qy);
-            acc[3].add(qz);
-            acc[4].add(mx);
-            acc[5].add(my);
-            acc[6].add(mz);
-            acc[7].add(qx * mx);
-            acc[8].add(qx * my);
-            acc[9].add(qx * mz);
-            acc[10].add(qy * mx);
-            acc[11].add(qy * my);
-            acc[12].add(qy * mz);
-            acc[13].add(qz * mx);
-            acc[14].add(qz * my);
-            acc[15].add(qz * mz);
-            acc[16].add(d);
-        }
-        // block reduction in FP64
-#pragma unroll
-        for (int k = 0; k < kNSum; ++k) {
-            double v = acc[k].value();
-            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) s_part[wid][k] = v;
-        }
-        __syncthreads();
-        // lane k of warp 0 totals sum k over the warps
-        if (wid == 0 && lane < kNSum) {
-            double v = 0;
-            for (int w = 0; w < kIcpThreads / 32; ++w) v += s_part[w][lane];
-            s_part[0][lane] = v;
-        }
-        __syncwarp();
-        if (tid == 0) {
-            double sum[kNSum];
-            for (int k = 0; k < kNSum; ++k) sum[k] = s_part[0][k];
-            const double cnt = sum[0];
-            if (cnt < 3) {
-                s_done = 2;  // too few correspondences: not converged
-            } else {
-                double R[9], t[3];
-                kabsch(cnt, sum + 1, sum + 4, sum + 7, R, t);
-                double Tn[16];
-                for (int i = 0; i < 3; ++i)
-                    for (int j = 0; j < 4; ++j)
-                        Tn[4 * i + j] = R[3 * i] * s_T[j] + R[3 * i + 1] * s_T[4 + j] + R[3 * i + 2] * s_T[8 + j] + (j == 3 ? t[i] : 0.0);
-                for (int j = 0; j < 4; ++j) Tn[12 + j] = s_T[12 + j];
-                for (int i = 0; i < 16; ++i) s_T[i] = Tn[i];
-                ++it;
-                const double cosang = 0.5 * (R[0] + R[4] + R[8] - 1.0);
-                const double tr2 = t[0] * t[0] + t[1] * t[1] + t[2] * t[2];
-                const double mse = sum[16] / cnt;
-                if (it >= prm.max_iter) s_done = 1;
-                else if (cosang >= 1.0 - (double)prm.transform_eps && tr2 <= (double)prm.transform_eps) s_done = 1;
-                else if (fabs(mse - s_prev) < (double)prm.mse_abs_eps) s_done = 1;
-                else if (fabs(mse - s_prev) / s_prev < (double)prm.fitness_eps) s_done = 1;
-                s_prev = mse;
+        search();
+        if (T == kIcpThreads || tid < kIcpThreads) {
+            KSum acc[kNSum];
+            for (uint32_t i = a + tid; i < b && !empty_t; i += kIcpThreads) {
+                float qx, qy, qz;
+                moved(i, qx, qy, qz);
+                float4 m;
+                const float d = nearest(i, qx, qy, qz, m);
+                if (d > corr2f) continue;
+                acc[0].add(1.f);
+                acc[1].add(qx);
+                acc[2].add(qy);
+                acc[3].add(qz);
+                acc[4].add(m.x);
+                acc[5].add(m.y);
+                acc[6].add(m.z);
+                acc[7].add(qx * m.x);
+                acc[8].add(qx * m.y);
+                acc[9].add(qx * m.z);
+                acc[10].add(qy * m.x);
+                acc[11].add(qy * m.y);
+                acc[12].add(qy * m.z);
+                acc[13].add(qz * m.x);
+                acc[14].add(qz * m.y);
+                acc[15].add(qz * m.z);
+                acc[16].add(d);
             }
+            // block reduction in FP64
+            double v[kNSum];
+#pragma unroll
+            for (int k = 0; k < kNSum; ++k) v[k] = acc[k].value();
+            int which;
+            const double sum = warp_sums17(v, lane, &which);
+            if (which >= 0) s_part[wid][which] = sum;
         }
         __syncthreads();
-        const int done = s_done;
-        if (done) {
+        if (wid == 0) {
+            const unsigned full = 0xffffffffu;
+            // lane k totals sum k over the warps
+            double v = 0;
+            if (lane < kNSum)
+                for (int w = 0; w < kIcpThreads / 32; ++w) v += s_part[w][lane];
+            const double cnt = __shfl_sync(full, v, 0);
+            int done = 0;
+            if (cnt < 3) {
+                done = 2;  // too few correspondences: not converged
+            } else {
+                // Kabsch: lane 3 i + j holds element (i, j) of the covariance
+                const int l9 = lane < 9 ? lane : 0, i = l9 / 3, j = l9 % 3;
+                const double cp = __shfl_sync(full, v, 1 + i) / cnt, cq = __shfl_sync(full, v, 4 + j) / cnt;
+                const double h = __shfl_sync(full, v, 7 + l9) - cnt * cp * cq;
+                double R;
+                if (!polar3(h, lane, &R)) {
+                    if (lane < 9) s_H[lane] = h;
+                    __syncwarp();
+                    if (lane == 0) kabsch_svd(s_H, s_R);
+                    __syncwarp();
+                    R = s_R[l9];
+                }
+                // t = cq - R cp, and T <- [R t] T: lane 4 r + c holds element (r, c)
+                const int l12 = lane < 12 ? lane : 0, rr = l12 / 4, c = l12 % 4;
+                const double R0 = __shfl_sync(full, R, 3 * rr), R1 = __shfl_sync(full, R, 3 * rr + 1),
+                             R2 = __shfl_sync(full, R, 3 * rr + 2);
+                const double t = __shfl_sync(full, cq, rr) - (R0 * __shfl_sync(full, cp, 0) + R1 * __shfl_sync(full, cp, 3) +
+                                                              R2 * __shfl_sync(full, cp, 6));
+                const double Tn = R0 * s_T[c] + R1 * s_T[4 + c] + R2 * s_T[8 + c] + (c == 3 ? t : 0.0);
+                __syncwarp();
+                if (lane < 12) s_T[lane] = Tn;
+                ++it;
+                const double cosang = 0.5 * (__shfl_sync(full, R, 0) + __shfl_sync(full, R, 4) + __shfl_sync(full, R, 8) - 1.0);
+                const double t0 = __shfl_sync(full, t, 0), t1 = __shfl_sync(full, t, 4), t2 = __shfl_sync(full, t, 8);
+                const double tr2 = t0 * t0 + t1 * t1 + t2 * t2;
+                const double mse = __shfl_sync(full, v, 16) / cnt;
+                if (it >= prm.max_iter) done = 1;
+                else if (cosang >= 1.0 - (double)prm.transform_eps && tr2 <= (double)prm.transform_eps) done = 1;
+                else if (fabs(mse - prev_mse) < (double)prm.mse_abs_eps) done = 1;
+                else if (fabs(mse - prev_mse) / prev_mse < (double)prm.fitness_eps) done = 1;
+                prev_mse = mse;
+            }
             conv = done == 1;
-            break;
+            if (lane == 0) s_done = done;
         }
+        first = false;
         __syncthreads();
+        if (s_done) break;
     }
     // fitness score of the final transform (getFitnessScore)
     if (tid < 12) s_Tf[tid] = (float)s_T[tid];
     __syncthreads();
-    KSum fs;
-    for (uint32_t i = a + tid; i < b && !empty_t; i += kIcpThreads) {
-        const float x = __ldg(src + 3ull * i), y = __ldg(src + 3ull * i + 1), z = __ldg(src + 3ull * i + 2);
-        const float qx = s_Tf[0] * x + s_Tf[1] * y + s_Tf[2] * z + s_Tf[3];
-        const float qy = s_Tf[4] * x + s_Tf[5] * y + s_Tf[6] * z + s_Tf[7];
-        const float qz = s_Tf[8] * x + s_Tf[9] * y + s_Tf[10] * z + s_Tf[11];
-        float mx, my, mz;
-        fs.add(grid_nn(g, cs, tsorted, tb, qx, qy, qz, &mx, &my, &mz));
+    search();
+    if (T == kIcpThreads || tid < kIcpThreads) {
+        KSum fs;
+        for (uint32_t i = a + tid; i < b && !empty_t; i += kIcpThreads) {
+            float qx, qy, qz;
+            moved(i, qx, qy, qz);
+            float4 m;
+            fs.add(nearest(i, qx, qy, qz, m));
+        }
+        double v = fs.value();
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) s_part[wid][0] = v;
     }
-    double v = fs.value();
-    for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) s_part[wid][0] = v;
     __syncthreads();
     if (tid == 0) {
         double tot = 0;
@@ -525,8 +692,7 @@ __global__ void __launch_bounds__(kIcpThreads) k_nn_mean(const float* __restrict
         const float qx = M[0] * x + M[1] * y + M[2] * z + M[3];
         const float qy = M[4] * x + M[5] * y + M[6] * z + M[7];
         const float qz = M[8] * x + M[9] * y + M[10] * z + M[11];
-        float mx, my, mz;
-        acc.add(grid_nn(g, cs, sorted, gb, qx, qy, qz, &mx, &my, &mz));
+        acc.add(grid_nn(g, cs, sorted + gb, qx, qy, qz, -1).d);
     }
     double v = acc.value();
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -853,9 +1019,17 @@ extern "C" int pvvc_icp_batch(int32_t npairs, const float* src_xyz, const uint32
     cudaStream_t s = (cudaStream_t)stream;
     if (!grid_attr_ready()) return PVVC_ERR_CUDA;
     k_grid<256><<<npairs, 256, kGridSmem, s>>>(tgt_xyz, tgt_off, nullptr, w.hdr, w.cstart, w.sorted, kIcpCellMul);
-    k_icp<<<npairs, kIcpThreads, 0, s>>>(src_xyz, src_off, tgt_off, w.hdr, w.cstart, w.sorted, kIcpCellMul, init, *params,
-                                         T_out, mse_out,
-                                         iters_out, converged_out);
+    // the source-side grid's place (pvvc_cloud_mse_batch's) holds the neighbours
+    // the source-side grid's place (pvvc_cloud_mse_batch's) holds the neighbours
+    const uint32_t nsrc = (uint32_t)std::min<uint64_t>(total_src_points, 0xFFFFFFFFu);
+    auto launch = [&](auto kernel, int threads) {
+        kernel<<<npairs, threads, 0, s>>>(src_xyz, src_off, tgt_off, w.hdr, w.cstart, w.sorted, init, *params, T_out, mse_out,
+                                          iters_out, converged_out, 0xFFFFFFFFu, w.cstart2, nsrc);
+    };
+    // (the figures stand at k_icp)
+    if (npairs <= 4 * sm_count()) launch(k_icp<true, 1024>, 1024);
+    else if (npairs <= 10 * sm_count()) launch(k_icp<true, 512>, 512);
+    else launch(k_icp<true, 256>, 256);
     return cudaGetLastError() == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;
 }
 
@@ -980,10 +1154,12 @@ extern "C" int pvvc_icp_batch_noalloc(int32_t npairs, const float* src_xyz, cons
     const float4* csorted = sorted;
     const GridHdr* chdr = hdr;
     pvvc_icp_params prm = *params;
+    int* no_j = nullptr;
+    uint32_t no_src = 0;
     void* ia[] = {(void*)&src_xyz, (void*)&src_off, (void*)&tgt_off, (void*)&chdr, (void*)&ccs, (void*)&csorted,
-                  (void*)&kmul, (void*)&init, (void*)&prm, (void*)&T_out, (void*)&mse_out, (void*)&iters_out,
-                  (void*)&converged_out, (void*)&cap};
-    if (cudaLaunchKernel((const void*)k_icp, dim3(npairs), dim3(kIcpThreads), ia, 0, s) != cudaSuccess)
+                  (void*)&init, (void*)&prm, (void*)&T_out, (void*)&mse_out, (void*)&iters_out,
+                  (void*)&converged_out, (void*)&cap, (void*)&no_j, (void*)&no_src};
+    if (cudaLaunchKernel((const void*)k_icp<false, kIcpThreads>, dim3(npairs), dim3(kIcpThreads), ia, 0, s) != cudaSuccess)
         return PVVC_ERR_CUDA;
     return PVVC_OK;
 }

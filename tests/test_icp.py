@@ -130,3 +130,54 @@ def test_gpu_icp_edge_cases(pvvc_lib):
     assert not conv[0] and not conv[1]          # fewer than 3 correspondences
     assert np.isfinite(T).all() and (iters <= 30).all()
     assert conv[3] and mse[3] < 1.0
+
+
+@pytest.mark.gpu
+def test_gpu_icp_same_for_any_cta_size(pvvc_lib):
+    """One batch of pairs, and the same pairs repeated until the launch takes
+    smaller CTAs: a pair's results do not depend on the batch, bit for bit; and
+    neither on the scratch for its neighbours (the entry point without one)."""
+    import ctypes as C
+    import torch
+    from pvvc import _lib as L
+    from pvvc.icp import IcpBatch, Pairs
+    base = _pairs(pvvc_lib, 12, 7)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    ref = None
+    for reps in (1, 4 * sms // 12 + 1, 10 * sms // 12 + 1):
+        p = Pairs(base.src * reps, base.tgt * reps, np.tile(base.T_true, (reps, 1, 1)))
+        b = IcpBatch(p)
+        b.run(max_iter=20)
+        T, mse, iters, conv = b.results()
+        got = (T.reshape(reps, 12, 16), mse.reshape(reps, 12), iters.reshape(reps, 12), conv.reshape(reps, 12))
+        ref = ref or [g[0] for g in got]
+        for g, w in zip(got, ref):
+            assert (g == w[None]).all()
+    b = IcpBatch(base)
+    prm = L.IcpParams(1e6, 20, 0.0, 0.0, 1e-6)
+    L.check(L.lib().pvvc_icp_batch_noalloc(b.n, b.src.data_ptr(), b.soff.data_ptr(), b.tgt.data_ptr(), b.toff.data_ptr(), None,
+                                           C.byref(prm), b.T.data_ptr(), b.mse.data_ptr(), b.iters.data_ptr(),
+                                           b.conv.data_ptr(), b.nt, torch.cuda.current_stream().cuda_stream), "noalloc")
+    for g, w in zip(b.results(), ref):
+        assert (g.reshape(w.shape) == w).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("flat", [1.0, 1e-3, 0.0])
+def test_gpu_icp_flat_patches(pvvc_lib, oracle, flat):
+    """A patch and its moved copy, flattened to a plane: the covariance's
+    smallest singular value goes to zero (the SVD takes over from the polar
+    iteration)."""
+    from pvvc.icp import IcpBatch, Pairs, rotation, rotation_error_deg
+    rng = np.random.default_rng(11)
+    s = np.unique(rng.integers(0, 60, (900, 3)), axis=0).astype(np.float64) * [1, 1, flat]
+    R = rotation([0, 0, 1], 1.0)
+    t = s @ R.T + [0.3, -0.2, 0.1 * flat]
+    p = Pairs([s.astype(np.float32)], [t.astype(np.float32)], np.eye(4)[None])
+    b = IcpBatch(p)
+    b.run(max_iter=30)
+    T, mse, _, _ = b.results()
+    To, fit, _, _ = oracle.icp_align(p.src[0], p.tgt[0], max_iter=30, fitness_eps=0.0, transform_eps=0.0, mse_abs_eps=1e-6)
+    assert rotation_error_deg(T, np.array([To]))[0] < ROT_TOL_DEG
+    assert _trans_err(T, np.array([To]), p)[0] < TRANS_TOL_VOX
+    assert abs(mse[0] - fit) <= MSE_RTOL * fit + 1e-3
