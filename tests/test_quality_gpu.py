@@ -64,3 +64,27 @@ def test_quality_empty_and_single(q, oracle):
     bc = np.array([[0, 0, 0], [11, 20, 30]], np.uint8)
     assert np.allclose(q.mse(a, ac, b, bc), oracle.cloud_quality(a, ac, b, bc), rtol=1e-7)
 
+
+
+@pytest.mark.parametrize("na,nb", [(1, 1), (255, 257), (256, 2), (4097, 511), (31, 9000)])
+def test_quality_block_edges(q, na, nb):
+    """Sizes around a block of queries and a scan block of cells, coarse grid
+    coordinates (many equal distances: the lower index wins) and a far outlier,
+    against brute force; the sums differ by their order only."""
+    rng = np.random.default_rng(na + nb)
+    a = rng.integers(0, 12, (na, 3)).astype(np.float32)
+    b = rng.integers(0, 12, (nb, 3)).astype(np.float32) + np.float32(0.5)
+    b[-1] += np.float32(5000.0)
+    ac = rng.integers(0, 256, (na, 3)).astype(np.uint8)
+    bc = rng.integers(0, 256, (nb, 3)).astype(np.uint8)
+    K = np.array([[0.299, 0.587, 0.114], [-0.168736, -0.331264, 0.5], [0.5, -0.418688, -0.081312]])
+
+    def side(p, pc, t, tc):
+        d = ((p[:, None].astype(np.float64) - t[None]) ** 2).sum(2)
+        j = d.argmin(1)  # the first of equal ones
+        e = (pc.astype(np.float64) - tc[j]) @ K.T
+        return [d.min(1).mean()] + list((e * e).mean(0))
+
+    want = np.stack([side(a, ac, b, bc), side(b, bc, a, ac)], 1).reshape(-1)
+    # the float YUV is off by at most 3 roundings of values below 512
+    assert np.allclose(q.mse(a, ac, b, bc), want, rtol=1e-5, atol=1e-4)
