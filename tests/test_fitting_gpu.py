@@ -49,3 +49,25 @@ def test_fitting_registered_gops_vs_oracle(fitter, oracle, pvvc_lib):
     for g in range(10):
         want, _ = oracle.fitting_cloud(gops[g], seed=seeds[g])
         assert np.array_equal(clouds[g].view(np.uint32), want.view(np.uint32)), g
+
+
+@pytest.mark.parametrize("patches,points,span", [
+    (1, 2, 9.0), (3, 1024, 60.0), (3, 1025, 60.0),   # the last cell on one CTA, the first on four; 1024 centroids staged at once
+    (12, 1024, 90.0), (12, 1025, 90.0),              # the last cell on four CTAs, the first on sixteen
+    (40, 77, 40.0), (300, 41, 40.0),                 # centroids of more than 32 and of more than 256 members
+    (5, 700, 0.0), (5, 3000, 0.0),                   # few distinct points: most centroids empty, redrawn
+])
+def test_fitting_cell_sizes(fitter, oracle, patches, points, span):
+    """One cell of patches * points points (the threshold above its extent),
+    the same bits as the oracle."""
+    rng = np.random.default_rng(patches * points)
+    if span:
+        pats = [rng.uniform(0, span, (points, 3)).astype(np.float32) for _ in range(patches)]
+    else:
+        pats = [rng.integers(0, 3, (points, 3)).astype(np.float32) for _ in range(patches)]
+    clouds, st = fitter.fit([pats], seeds=[3], clustering_ths=4096.0, max_iter=20)
+    want, ws = oracle.fitting_cloud(pats, seed=3, clustering_ths=4096.0, max_iter=20)
+    assert st["cells"] == 1 and want.shape[0] == points
+    assert (span == 0.0) == (st["empty_redraws"] > 0)
+    assert st["empty_redraws"] == ws["empty_redraws"] and st["iterations"] == min(ws["iterations"], 20)
+    assert np.array_equal(clouds[0].view(np.uint32), want.view(np.uint32))
