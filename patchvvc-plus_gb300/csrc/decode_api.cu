@@ -462,7 +462,7 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 const bool first = c0 == 0;
                 const bool phase_b = has_intra && !first;
                 if ((first && has_intra) || cnt >= p->tune.min_group) {
-                    GroupDesc g{slot_of[si], (int32_t)items.size(), cnt, (int16_t)((first && has_intra) ? 1 : 0)};
+                    GroupDesc g{slot_of[si], (int32_t)items.size(), cnt, (first && has_intra) ? 1 : 0};
                     items.insert(items.end(), L + c0, L + c0 + cnt);
                     (phase_b ? gb : ga).push_back(g);
                 } else {
@@ -471,8 +471,27 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 }
             }
         }
-        // Window groups: phase-A groups of at least kWinGroupMin slices, all
-        // of one size, in size tiers of whole groups (ga is already largest
+        // Which groups are small (k_raht_few).  While the batch has fewer groups
+        // that could be window groups than the device has SMs, all of them: their
+        // CTAs' lanes are busier and the long chains are the per-slice launch's.
+        // (GoPs of 20 and 30 frames: with 59 groups 0.62 and 0.67 ms, with window
+        // groups 0.80 and 0.85; with 177 groups 0.85 and 0.94, with window groups
+        // 0.83 and 0.86; with 464 groups 1.60 and 1.93, with window groups 1.24
+        // and 1.36.)
+        auto windowed = [&](const GroupDesc& g) {
+            bool ok = g.count >= kWinGroupMin;
+            for (int l = 1; ok && l < g.count; ++l) ok = W[items[g.first + l]].n == W[items[g.first]].n;
+            return ok;
+        };
+        const bool use_win = p->wide_only || std::count_if(ga.begin(), ga.end(), windowed) >= sm_count();
+        const int few_below = p->wide_only ? 0 : use_win ? kFewBelow : 33;
+        auto is_few = [&](const GroupDesc& g) { return g.count < few_below; };
+        // a launch's small groups after its others, their order kept; their count
+        auto few_last = [&](std::vector<GroupDesc>& v) {
+            return (int32_t)(v.end() - std::stable_partition(v.begin(), v.end(), [&](const GroupDesc& g) { return !is_few(g); }));
+        };
+        // Window groups (while there are enough, as above): phase-A groups of at
+        // least kWinGroupMin slices, all of one size, in size tiers of whole groups (ga is already largest
         // first), so a tier's inverse RAHT waits for its own RLGR only.  The
         // long tier's slices -- the critical path -- are decoded by the
         // per-slice long launch, whose iterations are the cheapest, into
@@ -483,11 +502,8 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         p->nwin_slices = 0;
         {
             std::vector<GroupDesc> gw, gr;
-            for (const GroupDesc& g : ga) {
-                bool ok = g.count >= kWinGroupMin;
-                for (int l = 1; ok && l < g.count; ++l) ok = W[items[g.first + l]].n == W[items[g.first]].n;
-                (ok ? gw : gr).push_back(g);
-            }
+            if (use_win)
+                for (const GroupDesc& g : ga) (windowed(g) ? gw : gr).push_back(g);
             if (!gw.empty()) {
                 const int nw = (int)gw.size();
                 p->nwin = nw;
@@ -502,6 +518,9 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 if (p->ngroups_a_long > 0 && p->side.ensure(true) != cudaSuccess) return PVVC_ERR_CUDA;
                 if (p->ngroups_a_mid > 0 && p->side2.ensure() != cudaSuccess) return PVVC_ERR_CUDA;
                 if (p->ngroups_a_mid2 > 0 && p->side3.ensure() != cudaSuccess) return PVVC_ERR_CUDA;
+                p->nfew[kSegLong] = p->ngroups_a_long;  // decoded into planes of their own, as small groups are
+                p->nfew[kSegMid] = p->nfew[kSegMid2] = 0;
+                p->nfew[kSegRest] = few_last(gr);
                 ga = gw;
                 ga.insert(ga.end(), gr.begin(), gr.end());
                 // RLGR order: the window groups' slices in group order (sizes
@@ -534,6 +553,7 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 std::vector<uint8_t> tier(n, 0);
                 for (int i = 0; i < p->nlong + p->nmid; ++i) tier[p->order[i]] = i < p->nlong ? 2 : 1;
                 std::vector<GroupDesc> gl, gm, gs;
+                p->nfew[kSegMid2] = 0;
                 for (const GroupDesc& g : ga) {
                     int t = 0;
                     for (int l = 0; l < g.count; ++l) t = std::max<int>(t, tier[items[g.first + l]]);
@@ -542,24 +562,17 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 p->ngroups_a_long = (int32_t)gl.size();
                 p->ngroups_a_mid = (int32_t)gm.size();
                 p->ngroups_a_mid2 = 0;
+                p->nfew[kSegLong] = few_last(gl);
+                p->nfew[kSegMid] = few_last(gm);
+                p->nfew[kSegRest] = few_last(gs);
                 ga = gl;
                 ga.insert(ga.end(), gm.begin(), gm.end());
                 ga.insert(ga.end(), gs.begin(), gs.end());
             }
         }
+        p->nfew[kSegB] = few_last(gb);
         p->groups = ga;
         p->groups.insert(p->groups.end(), gb.begin(), gb.end());
-        p->long_split_off = (int32_t)p->groups.size();
-        p->nlong_split = 0;
-        if (p->nwin > 0 && kLongSplit > 1)
-            for (int gi = 0; gi < p->ngroups_a_long; ++gi)
-                for (int h = 0; h < kLongSplit; ++h) {
-                    GroupDesc g = ga[gi];
-                    g.part = (uint8_t)h;
-                    g.parts = (uint8_t)kLongSplit;
-                    p->groups.push_back(g);
-                    ++p->nlong_split;
-                }
         p->ngroups_a = (int32_t)ga.size();
         p->ngroups_b = (int32_t)gb.size();
         p->idx = items;
@@ -569,13 +582,30 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         p->idx.insert(p->idx.end(), lb.begin(), lb.end());
         p->nlist_a = (int32_t)la.size();
         p->nlist_b = (int32_t)lb.size();
-        // coefficient regions: a group shares one frame-interleaved region
-        // (stride 32), every other slice owns contiguous planes
+        // coefficient regions: a group of k_raht_group shares one frame-interleaved
+        // region (stride 32), every other slice owns contiguous planes
         // (window groups first; a region holds the largest slice of its group)
+        auto is_small = [&](int gi) {
+            return is_few(p->groups[gi]) || (p->nwin > 0 && gi < p->ngroups_a_long);
+        };
         uint64_t c = 0;
         p->coef_win_floats = 0;
-        for (int32_t gi = 0; gi < p->ngroups_a + p->ngroups_b; ++gi) {  // (not the long groups' split copies)
+        uint64_t few_max = 1;  // points of a small group's slices
+        uint32_t wide_max = 1;  // of a slice of another group
+        for (int32_t gi = 0; gi < p->ngroups_a + p->ngroups_b; ++gi) {
             const GroupDesc& g = p->groups[gi];
+            if (is_small(gi)) {
+                for (int l = 0; l < g.count; ++l) {
+                    SliceWork& w = W[p->idx[g.first + l]];
+                    w.coef_off = c;
+                    w.coef_stride = 1;
+                    w.coef_lane = 0;
+                    c += 3ull * w.n;
+                    few_max = std::max(few_max, (uint64_t)g.count * w.n);
+                }
+                continue;
+            }
+            c = align_up(c, 32);  // a region's rows are whole 128-byte lines (vector stores, prefetches)
             uint32_t gn = 0;
             for (int l = 0; l < g.count; ++l) {
                 SliceWork& w = W[p->idx[g.first + l]];
@@ -585,6 +615,7 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 gn = std::max(gn, w.n);
             }
             c += 3ull * gn * 32;
+            wide_max = std::max(wide_max, gn);
             if ((int32_t)gi + 1 == p->nwin) p->coef_win_floats = c;
         }
         for (int li = p->list_a_off; li < (int)p->idx.size(); ++li) {
@@ -596,6 +627,8 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         }
         coef = c;
         p->coef_floats = coef;
+        p->grp_floats = 2ull * wide_max * 96;
+        p->few_floats = 6ull * few_max;
         // the prefix of the planes that the long-slice RLGR launch writes
         // (its groups come first; a long slice outside a group extends it)
         p->coef_long_floats = 0;
@@ -623,25 +656,34 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
     // group kernel: per persistent CTA two level buffers of [width][32 lanes][3]
     // floats; an internal level of a valid tree is never wider than its leaves
     {
-        uint32_t maxn = 0;
-        for (const auto& g : p->groups) maxn = std::max(maxn, W[p->idx[g.first]].n);
-        p->grp_ctas = std::min<int32_t>(p->ngroups_a + p->ngroups_b, p->tune.group_ctas_per_sm * sm_count());
-        p->grp_floats = 2ull * std::max<uint32_t>(maxn, 1) * 96;
+        const int32_t* nf = p->nfew;
+        const int32_t few_a = nf[kSegLong] + nf[kSegMid] + nf[kSegMid2] + nf[kSegRest];
+        const int32_t nwide = p->ngroups_a + p->ngroups_b - few_a - nf[kSegB];
+        p->grp_ctas = std::min<int32_t>(nwide, p->tune.group_ctas_per_sm * sm_count());
         p->ws_grp = off;
         off = align_up(off + 4ull * p->grp_floats * std::max(p->grp_ctas, 1), 256);
         // the long-slice groups run beside the others, with level buffers of their own
-        const int32_t nlg = p->nlong_split > 0 ? p->nlong_split : p->ngroups_a_long;  // the long groups' launch
-        p->grp_ctas_long = nlg > 0 ? std::min<int32_t>(nlg, p->grp_ctas) : 0;
+        p->grp_ctas_long = std::min<int32_t>(p->ngroups_a_long - nf[kSegLong], p->grp_ctas);
         p->ws_grp_long = off;
         off = align_up(off + 4ull * p->grp_floats * p->grp_ctas_long, 256);
-        p->grp_ctas_mid = p->ngroups_a_mid > 0 ? std::min<int32_t>(p->ngroups_a_mid, p->grp_ctas) : 0;
+        p->grp_ctas_mid = std::min<int32_t>(p->ngroups_a_mid - nf[kSegMid], p->grp_ctas);
         p->ws_grp_mid = off;
         off = align_up(off + 4ull * p->grp_floats * p->grp_ctas_mid, 256);
         p->grp_ctas_mid2 = p->ngroups_a_mid2 > 0 ? std::min<int32_t>(p->ngroups_a_mid2, p->grp_ctas) : 0;
         p->ws_grp_mid2 = off;
         off = align_up(off + 4ull * p->grp_floats * p->grp_ctas_mid2, 256);
+        // the small groups' level buffers: per CTA two of [slice][node][yuv]
+        const int32_t slots = kFewCtasPerSm * sm_count();
+        auto parts_of = [&](int32_t n) { return n > 0 ? std::min(kFewParts, std::max(1, slots / n)) : 1; };
+        p->few_parts_a = parts_of(few_a);
+        p->few_parts_b = parts_of(nf[kSegB]);
+        for (int i = 0; i < kSegs; ++i) {
+            p->few_ctas[i] = std::min<int32_t>(nf[i] * (i == kSegB ? p->few_parts_b : p->few_parts_a), slots);
+            p->ws_few[i] = off;
+            off = align_up(off + 4ull * p->few_floats * p->few_ctas[i], 256);
+        }
         p->ws_counter = off;
-        off = align_up(off + 32, 256);
+        off = align_up(off + 64, 256);
     }
     p->ws_bytes = std::max<uint64_t>(off, 256);
     lap(3);  // workspace layout
@@ -693,12 +735,26 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
         return PVVC_ERR_CUDA;
     }
     float* gsc = reinterpret_cast<float*>(w + p->ws_grp);
-    int* cnt = reinterpret_cast<int*>(w + p->ws_counter);  // queue counters: A long, B, A short, A medium, A medium 2
+    int* cnt = reinterpret_cast<int*>(w + p->ws_counter);  // queue counters: two per launch of groups
     const GroupDesc* dg = static_cast<const GroupDesc*>(p->d_groups.p);
     const int32_t* di = static_cast<const int32_t*>(p->d_idx.p);
-    auto raht_groups = [&](int first, int count, int* counter, float* scratch, int ctas, cudaStream_t on) {
-        return count <= 0 || launch_raht_group(dw, dg + first, count, di, st->v, coef, ts, rs, fs, xyz, rgb, p24, status,
-                                               scratch, p->grp_floats, ctas, counter, on) == cudaSuccess;
+    // `count` groups, the seg's small ones last
+    auto raht_groups = [&](int seg, int first, int count, float* scratch, int ctas, cudaStream_t on) {
+        const int few = p->nfew[seg], wide = count - few;
+        return launch_raht_group(dw, dg + first, wide, di, st->v, coef, ts, rs, fs, xyz, rgb, p24, status, scratch,
+                                 p->grp_floats, ctas, cnt + 2 * seg, on) == cudaSuccess &&
+               launch_raht_few(dw, dg + first + wide, few, seg == kSegB ? p->few_parts_b : p->few_parts_a, di, st->v, coef, ts,
+                               rs, fs, xyz, rgb, p24, status, reinterpret_cast<float*>(w + p->ws_few[seg]), p->few_floats,
+                               p->few_ctas[seg], cnt + 2 * seg + 1, on) == cudaSuccess;
+    };
+    // every phase-A group, on the main stream
+    auto raht_all = [&] {
+        int at = 0;
+        const int count[4] = {p->ngroups_a_long, p->ngroups_a_mid, p->ngroups_a_mid2,
+                              p->ngroups_a - p->ngroups_a_long - p->ngroups_a_mid - p->ngroups_a_mid2};
+        for (int i = 0; i < 4; at += count[i++])
+            if (!raht_groups(i, at, count[i], gsc, p->grp_ctas, s)) return false;
+        return true;
     };
     auto clear = [&](uint64_t from, uint64_t to) {
         return to <= from || cudaMemsetAsync(coef + from, 0, 4ull * (to - from), s) == cudaSuccess;
@@ -742,27 +798,24 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
             if ((nl > 0 && (cudaEventRecord(L.join, L.s) != cudaSuccess || cudaStreamWaitEvent(s, L.join, 0) != cudaSuccess)) ||
                 (nm > 0 && (cudaEventRecord(M.join, M.s) != cudaSuccess || cudaStreamWaitEvent(s, M.join, 0) != cudaSuccess)) ||
                 (nm2 > 0 && (cudaEventRecord(M2.join, M2.s) != cudaSuccess || cudaStreamWaitEvent(s, M2.join, 0) != cudaSuccess)) ||
-                !mark(2) || !raht_groups(0, p->ngroups_a, cnt, gsc, p->grp_ctas, s))
+                !mark(2) || !raht_all())
                 return PVVC_ERR_CUDA;
         } else {
-            // the long groups, each split over several CTAs (their copies after the phase-B groups)
-            const int lf = p->nlong_split > 0 ? p->long_split_off : 0, ln = p->nlong_split > 0 ? p->nlong_split : nl;
             if (nl > 0 && ((tree_aside && cudaStreamWaitEvent(L.s, p->tree.mid, 0) != cudaSuccess) ||
-                           !raht_groups(lf, ln, cnt, reinterpret_cast<float*>(w + p->ws_grp_long), p->grp_ctas_long, L.s) ||
+                           !raht_groups(kSegLong, 0, nl, reinterpret_cast<float*>(w + p->ws_grp_long), p->grp_ctas_long, L.s) ||
                            cudaEventRecord(L.join, L.s) != cudaSuccess))
                 return PVVC_ERR_CUDA;
             if (nm > 0 && ((tree_aside && cudaStreamWaitEvent(M.s, p->tree.mid, 0) != cudaSuccess) ||
-                           !raht_groups(nl, nm, cnt + 3, reinterpret_cast<float*>(w + p->ws_grp_mid), p->grp_ctas_mid,
-                                        M.s) ||
+                           !raht_groups(kSegMid, nl, nm, reinterpret_cast<float*>(w + p->ws_grp_mid), p->grp_ctas_mid, M.s) ||
                            cudaEventRecord(M.join, M.s) != cudaSuccess))
                 return PVVC_ERR_CUDA;
             if (nm2 > 0 && ((tree_aside && cudaStreamWaitEvent(M2.s, p->tree.mid, 0) != cudaSuccess) ||
-                            !raht_groups(nl + nm, nm2, cnt + 4, reinterpret_cast<float*>(w + p->ws_grp_mid2),
+                            !raht_groups(kSegMid2, nl + nm, nm2, reinterpret_cast<float*>(w + p->ws_grp_mid2),
                                          p->grp_ctas_mid2, M2.s) ||
                             cudaEventRecord(M2.join, M2.s) != cudaSuccess))
                 return PVVC_ERR_CUDA;
             if ((tree_aside && cudaStreamWaitEvent(s, p->tree.mid, 0) != cudaSuccess) ||
-                !raht_groups(ns0, p->ngroups_a - ns0, cnt + 2, gsc, p->grp_ctas, s) ||
+                !raht_groups(kSegRest, ns0, p->ngroups_a - ns0, gsc, p->grp_ctas, s) ||
                 (nl > 0 && cudaStreamWaitEvent(s, L.join, 0) != cudaSuccess) ||
                 (nm > 0 && cudaStreamWaitEvent(s, M.join, 0) != cudaSuccess) ||
                 (nm2 > 0 && cudaStreamWaitEvent(s, M2.join, 0) != cudaSuccess))
@@ -774,7 +827,7 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
             launch_rlgr(dw, ord, p->nslices, payload, coef, rs, p->tune.rlgr_block, 0, s) != cudaSuccess || !mark(2))
             return PVVC_ERR_CUDA;
         if (tree_aside && cudaStreamWaitEvent(s, p->tree.mid, 0) != cudaSuccess) return PVVC_ERR_CUDA;
-        if (!raht_groups(0, p->ngroups_a, cnt, gsc, p->grp_ctas, s)) return PVVC_ERR_CUDA;
+        if (!raht_all()) return PVVC_ERR_CUDA;
     } else {
         // Size tiers, largest first in `order`: the long slices on SMs of their
         // own (stream `side`), the medium ones (stream `side2`), the rest (this
@@ -799,7 +852,7 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
             // stage markers: every tier decoded, then every group
             if (cudaEventRecord(L.join, L.s) != cudaSuccess || cudaStreamWaitEvent(s, L.join, 0) != cudaSuccess ||
                 (nm > 0 && cudaStreamWaitEvent(s, M.mid, 0) != cudaSuccess) || !mark(2) ||
-                !raht_groups(0, p->ngroups_a, cnt, gsc, p->grp_ctas, s))
+                !raht_all())
                 return PVVC_ERR_CUDA;
         } else {
             // Each tier's groups follow its decode on its stream.  A group can
@@ -808,16 +861,15 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
             if (tree_aside && cudaStreamWaitEvent(s, p->tree.mid, 0) != cudaSuccess) return PVVC_ERR_CUDA;
             if (cudaEventRecord(L.mid, s) != cudaSuccess) return PVVC_ERR_CUDA;  // the small tier decoded, trees built
             if (nm > 0 && (cudaStreamWaitEvent(M.s, L.mid, 0) != cudaSuccess ||
-                           !raht_groups(na_l, na_m, cnt + 3, reinterpret_cast<float*>(w + p->ws_grp_mid), p->grp_ctas_mid,
-                                        M.s) ||
+                           !raht_groups(kSegMid, na_l, na_m, reinterpret_cast<float*>(w + p->ws_grp_mid), p->grp_ctas_mid, M.s) ||
                            cudaEventRecord(M.join, M.s) != cudaSuccess))
                 return PVVC_ERR_CUDA;
             if (cudaStreamWaitEvent(L.s, L.mid, 0) != cudaSuccess ||
                 (nm > 0 && cudaStreamWaitEvent(L.s, M.mid, 0) != cudaSuccess) ||
-                !raht_groups(0, na_l, cnt, reinterpret_cast<float*>(w + p->ws_grp_long), p->grp_ctas_long, L.s) ||
+                !raht_groups(kSegLong, 0, na_l, reinterpret_cast<float*>(w + p->ws_grp_long), p->grp_ctas_long, L.s) ||
                 cudaEventRecord(L.join, L.s) != cudaSuccess)
                 return PVVC_ERR_CUDA;
-            if (!raht_groups(na_l + na_m, na_s, cnt + 2, gsc, p->grp_ctas, s) ||
+            if (!raht_groups(kSegRest, na_l + na_m, na_s, gsc, p->grp_ctas, s) ||
                 cudaStreamWaitEvent(s, L.join, 0) != cudaSuccess || (nm > 0 && cudaStreamWaitEvent(s, M.join, 0) != cudaSuccess))
                 return PVVC_ERR_CUDA;
         }
@@ -828,8 +880,7 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
         !mark(3))
         return PVVC_ERR_CUDA;
     // phase B: predictive slices whose intra colours phase A produced
-    if (launch_raht_group(dw, dg + p->ngroups_a, p->ngroups_b, di, st->v, coef, ts, rs, fs, xyz, rgb, p24, status, gsc,
-                          p->grp_floats, p->grp_ctas, cnt + 1, s) != cudaSuccess ||
+    if (!raht_groups(kSegB, p->ngroups_a, p->ngroups_b, gsc, p->grp_ctas, s) ||
         launch_raht_slice(dw, di + p->list_b_off, p->nlist_b, st->v, coef, fb, ts, rs, fs, xyz, rgb, p24, status, kRahtWcap, s) !=
             cudaSuccess ||
         !mark(4))
@@ -950,20 +1001,16 @@ extern "C" int pvvc_plan_info_get(const pvvc_plan* p, pvvc_plan_info* info) {
         p->nwin > 0
             ? 4ull * p->coef_long_floats + (p->nslices > p->nwin_slices ? 4ull * (p->coef_floats - p->coef_win_floats) : 0ull)
             : 4ull * p->coef_floats;
-    if (p->nslices > 0 && p->nwin > 0)
-        info->kernels = (p->nintra > 0) + (p->ngroups_a_long > 0) + (p->ngroups_a_mid > 0) + (p->ngroups_a_mid2 > 0) +
-                        (p->nwin > p->ngroups_a_long + p->ngroups_a_mid + p->ngroups_a_mid2) +
-                        (p->nslices > p->nwin_slices) + (p->ngroups_a_long > 0) + (p->ngroups_a_mid > 0) +
-                        (p->ngroups_a_mid2 > 0) +
-                        (p->ngroups_a > p->ngroups_a_long + p->ngroups_a_mid + p->ngroups_a_mid2) + (p->nlist_a > 0) +
-                        (p->ngroups_b > 0) +
-                        (p->nlist_b > 0);
-    else if (p->nslices > 0)
-        info->kernels = (p->nintra > 0) + 1 + (p->nlong > 0) + (p->nmid > 0) +
-                        (p->nlong > 0 ? (p->ngroups_a_long > 0) + (p->ngroups_a_mid > 0) +
-                                            (p->ngroups_a > p->ngroups_a_long + p->ngroups_a_mid)
-                                      : (p->ngroups_a > 0)) +
-                        (p->nlist_a > 0) + (p->ngroups_b > 0) + (p->nlist_b > 0);
+    if (p->nslices > 0) {
+        const int32_t first3 = p->ngroups_a_long + p->ngroups_a_mid + p->ngroups_a_mid2;
+        const int32_t count[kSegs] = {p->ngroups_a_long, p->ngroups_a_mid, p->ngroups_a_mid2, p->ngroups_a - first3,
+                                      p->ngroups_b};
+        int32_t k = (p->nintra > 0) + (p->nlist_a > 0) + (p->nlist_b > 0);
+        for (int i = 0; i < kSegs; ++i) k += (count[i] > p->nfew[i]) + (p->nfew[i] > 0);
+        info->kernels = k + (p->nwin > 0 ? (p->ngroups_a_long > 0) + (p->ngroups_a_mid > 0) + (p->ngroups_a_mid2 > 0) +
+                                               (p->nwin > first3) + (p->nslices > p->nwin_slices)
+                                         : 1 + (p->nlong > 0) + (p->nmid > 0));
+    }
     return PVVC_OK;
 }
 

@@ -33,6 +33,10 @@ cudaError_t launch_refresh(SliceWork* work, int n, const CallFields& f, cudaStre
 cudaError_t launch_raht_slice(const SliceWork* work, const int32_t* list, int count, const StateView& st, const float* coef,
                               float* fallback, const int32_t* tstatus, const int32_t* rstatus, int32_t* fstatus, float* xyz,
                               uint8_t* rgb, float* p24, int32_t* status, int wcap, cudaStream_t s);
+cudaError_t launch_raht_few(const SliceWork* work, const GroupDesc* groups, int ngroups, int parts, const int32_t* items,
+                            const StateView& st, const float* coef, const int32_t* tstatus, const int32_t* rstatus,
+                            int32_t* fstatus, float* xyz, uint8_t* rgb, float* p24, int32_t* status, float* scratch,
+                            uint64_t scratch_floats, int nctas, int* counter, cudaStream_t s);
 cudaError_t launch_raht_group(const SliceWork* work, const GroupDesc* groups, int ngroups, const int32_t* items,
                               const StateView& st, const float* coef, const int32_t* tstatus, const int32_t* rstatus,
                               int32_t* fstatus, float* xyz, uint8_t* rgb, float* p24, int32_t* status, float* scratch,
@@ -51,9 +55,10 @@ constexpr int kRlgrLongLanes = 32;
 // has at least kMidSplitMin groups
 constexpr int kMidSplit = 2;
 constexpr int kMidSplitMin = 64;
-// window mode: the long tier's groups (the largest, the last to finish)
-// are inverse-transformed by kLongSplit CTAs each
-constexpr int kLongSplit = 2;
+// k_raht_few: its CTAs per SM, and the most CTAs a group is split over (so many
+// that the phase's groups fill the device)
+constexpr int kFewCtasPerSm = 2;
+constexpr int kFewParts = 8;
 
 // the SM count (queried once)
 inline int sm_count() {
@@ -138,6 +143,9 @@ struct HostBuf {  // pinned, grow-only
 };
 }  // namespace pvvc
 
+// the launches of grouped inverse transforms of a plan
+enum { kSegLong, kSegMid, kSegMid2, kSegRest, kSegB, kSegs };
+
 struct pvvc_plan {
     pvvc_tune tune{};  // resolved launch shapes
     double host_ms[5] = {};  // host time of the last build's stages (pvvc_plan_host_times)
@@ -149,9 +157,13 @@ struct pvvc_plan {
     uint64_t ws_grp_long = 0, ws_grp_mid = 0;  // level buffers of the long and medium groups' launches
     int32_t grp_ctas_mid2 = 0;
     uint64_t ws_grp_mid2 = 0;
-    // window mode: the long tier's groups again, each split over
-    // kLongSplit CTAs for their inverse transform (after the phase-B groups)
-    int32_t long_split_off = 0, nlong_split = 0;
+    // The groups of a launch (phase A's long, medium, medium 2 and other groups,
+    // phase B's): the small ones come last and have a launch of their own
+    // (k_raht_few), each over few_parts_a or _b CTAs.
+    bool wide_only = false;  // no such split (set before the build)
+    int32_t nfew[kSegs] = {}, few_ctas[kSegs] = {};
+    int32_t few_parts_a = 1, few_parts_b = 1;
+    uint64_t ws_few[kSegs] = {}, few_floats = 0;  // their level buffers
     uint64_t coef_floats = 0;
     uint64_t coef_long_floats = 0;  // planes prefix the long-slice RLGR launch writes
     uint64_t coef_mid_floats = 0;   // ... and the medium tier

@@ -885,9 +885,9 @@ __device__ __forceinline__ uint8_t to_u8(float v) {
     return (uint8_t)__float2uint_rd(__fadd_rd(c, 0.5f));
 }
 
-// one leaf: reference add / store, YUV->RGB, transform, output
-__device__ __forceinline__ void emit_leaf(const SliceWork& w, const StateView& st, size_t lb, uint32_t leaf, float y,
-                                          float u, float v, bool predict, const OutPtrs& o) {
+// one leaf: reference add / store, YUV->RGB, transform (rows m), output
+__device__ __forceinline__ void emit_leaf(const float* m, uint64_t out_off, bool white, const StateView& st, size_t lb,
+                                          uint32_t leaf, float y, float u, float v, bool predict, const OutPtrs& o) {
     float* ref = st.ref + (lb + leaf) * 3;
     if (predict) {
         y = __fadd_rn(y, ref[0]);
@@ -900,7 +900,6 @@ __device__ __forceinline__ void emit_leaf(const SliceWork& w, const StateView& s
     }
     const float* p = st.xyz + (lb + leaf) * 3;
     const float x0 = p[0], y0 = p[1], z0 = p[2];
-    const float* m = w.mv;
     const float X = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(x0, m[0]), __fmul_rn(y0, m[1])), __fmul_rn(z0, m[2])), m[3]);
     const float Y = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(x0, m[4]), __fmul_rn(y0, m[5])), __fmul_rn(z0, m[6])), m[7]);
     const float Z = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(x0, m[8]), __fmul_rn(y0, m[9])), __fmul_rn(z0, m[10])), m[11]);
@@ -908,7 +907,7 @@ __device__ __forceinline__ void emit_leaf(const SliceWork& w, const StateView& s
     const float R = __fadd_rn(y, __fmul_rn(1.4020f, dv));
     const float G = __fsub_rn(__fsub_rn(y, __fmul_rn(0.3441f, du)), __fmul_rn(0.7141f, dv));
     const float B = __fadd_rn(y, __fmul_rn(1.7720f, du));
-    const uint64_t oi = w.out_off + leaf;
+    const uint64_t oi = out_off + leaf;
     if (o.xyz) {
         o.xyz[oi * 3 + 0] = X;
         o.xyz[oi * 3 + 1] = Y;
@@ -921,7 +920,6 @@ __device__ __forceinline__ void emit_leaf(const SliceWork& w, const StateView& s
     }
     if (o.p24) {  // CUDA2OpenGL.cu:44-58: unrounded /255, patches under 10 points white
         float* q = o.p24 + oi * 6;
-        const bool white = w.n < 10;
         q[0] = X;
         q[1] = Y;
         q[2] = Z;
@@ -1027,7 +1025,7 @@ __global__ void __launch_bounds__(T) k_raht_slice(const SliceWork* __restrict__ 
     const float* cu = cy + N;
     const float* cv = cu + N;
     if (H == 1) {
-        if (tid == 0) emit_leaf(w, st, lb, 0, cy[0], cu[0], cv[0], predict, o);
+        if (tid == 0) emit_leaf(w.mv, w.out_off, w.n < 10, st, lb, 0, cy[0], cu[0], cv[0], predict, o);
         return;
     }
     float *gA, *gB;
@@ -1063,7 +1061,7 @@ __global__ void __launch_bounds__(T) k_raht_slice(const SliceWork* __restrict__ 
                     gB[3 * child + 1] = ou[c];
                     gB[3 * child + 2] = ov[c];
                 } else {
-                    emit_leaf(w, st, lb, child, oy[c], ou[c], ov[c], predict, o);
+                    emit_leaf(w.mv, w.out_off, w.n < 10, st, lb, child, oy[c], ou[c], ov[c], predict, o);
                 }
             }
         }
@@ -1150,7 +1148,9 @@ struct NodeRows {
     float2 ab[7][kRowNodes];
 };
 
-// k_raht_group: persistent CTAs; each takes the next group of slices that
+// k_raht_group (window groups: near 32 slices each, as many as the device has SMs
+// or more; there its uniform control flow and line-wide accesses cost the least
+// instructions a point): persistent CTAs; each takes the next group of slices that
 // share a slot (the frames of one patch) from a queue.  Lane f of every warp
 // owns frame f (same control flow in all lanes, node records are broadcast
 // loads).  The intra slice, when the group has one, is lane 0 and hands its
@@ -1341,7 +1341,7 @@ __global__ void __launch_bounds__(32 * kGrpWarps, 3) k_raht_group(const SliceWor
                 __syncwarp();
             };
             if (H == 1) {
-                if (wid == 0 && G.part == 0) {
+                if (wid == 0) {
                     const float gy = act ? cy[0] : 0.f, gu = act ? cu[0] : 0.f, gv = act ? cv[0] : 0.f;
                     finish(0, 0, gy, gu, gv);
                     flush(0, 1);
@@ -1429,11 +1429,9 @@ __global__ void __launch_bounds__(32 * kGrpWarps, 3) k_raht_group(const SliceWor
                         }
                     }
                 };
-                // this warp's share of the last-level nodes: of all the
-                // warps of the CTAs the group is split over
-                const int parts = G.parts > 1 ? G.parts : 1, vw = G.part * kGrpWarps + wid;
-                const int per = (cnt + kGrpWarps * parts - 1) / (kGrpWarps * parts);
-                const int j0 = min(cnt, vw * per), j1 = min(cnt, j0 + per);
+                // this warp's share of the last-level nodes
+                const int per = (cnt + kGrpWarps - 1) / kGrpWarps;
+                const int j0 = min(cnt, wid * per), j1 = min(cnt, j0 + per);
                 uint32_t base = 0, staged = 0;
                 int pj = 0;
                 if (j0 < j1) {
@@ -1497,6 +1495,246 @@ __global__ void __launch_bounds__(32 * kGrpWarps, 3) k_raht_group(const SliceWor
                     }
                 }
                 if (staged) flush(base, staged);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// k_raht_few: groups of slices that share a slot, `parts` CTAs a group, each
+// taking a range of the last internal level's nodes and their ancestors.  A warp
+// takes 32 consecutive nodes of a level, a lane each, and holds their records
+// while it goes through (some of) the slices, whose planes are contiguous: the
+// lanes are as full as the level is wide, where k_raht_group's lane per slice
+// leaves 32 - count of them idle, and there are 3 n floats a slice to clear
+// instead of 96 n a group.  The level signal is [slice][node][yuv] in the CTA's
+// scratch region.  The leaves of 32 nodes are contiguous: their colours go
+// through the warp's shared rows, then a lane writes a point.  At the last
+// internal level the intra slice, when the group has one, goes first: the others
+// read its colours.
+//
+// 58 groups of 8 slices (0.8M points): k_raht_group took 275 us for its long tier
+// (22 CTAs, 8 of 32 lanes), this 36 (110 CTAs); 1,023 groups of 2 (4M points): 728
+// us for the medium tier, 81; the long tier of a 30-frame GoP (64 groups of 30,
+// 8M points): 535 us over two CTAs a group, 350 here.  A pair of (slice, node) a
+// thread writing its own leaves took 492 on that tier: 12-byte stores 48 bytes
+// apart, half the lanes idle.  Bound by the instructions of the transform and the
+// points (some 10 a point) at two CTAs an SM.
+constexpr int kFewThreads = 256;
+constexpr int kFewWarps = kFewThreads / 32;
+
+// a node's record in a lane's registers (no children, no coefficients: idle)
+struct LaneNode {
+    uint32_t byte, cb, m, ci;
+    float2 ab[7];
+};
+
+__device__ __forceinline__ void lane_inverse(const LaneNode& r, const float* cy, uint32_t N, float gy, float gu, float gv,
+                                             float (&oy)[8], float (&ou)[8], float (&ov)[8]) {
+    const float *cu = cy + N, *cv = cu + N;
+    float hy[8], hu[8], hv[8];
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        const uint32_t k = r.ci + __popc(r.m & ((1u << i) - 2u));
+        const bool coded = r.m & (1u << i);
+        hy[i] = coded ? __ldg(cy + k) : 0.f;
+        hu[i] = coded ? __ldg(cu + k) : 0.f;
+        hv[i] = coded ? __ldg(cv + k) : 0.f;
+    }
+    float sy[8], su[8], sv[8];
+    sy[1] = gy;
+    su[1] = gu;
+    sv[1] = gv;
+#pragma unroll
+    for (int i = 1; i < 8; ++i) {
+        const float2 t = r.ab[i - 1];
+        const float ay = sy[i], au = su[i], av = sv[i], nbv = -t.y;
+        // [G;H] = [[a,-b],[b,a]] [g;h]   (InvertHaarTransform, octree_base.cc:186-206)
+        const float Gy = __fadd_rn(__fmul_rn(ay, t.x), __fmul_rn(hy[i], nbv));
+        const float Gu = __fadd_rn(__fmul_rn(au, t.x), __fmul_rn(hu[i], nbv));
+        const float Gv = __fadd_rn(__fmul_rn(av, t.x), __fmul_rn(hv[i], nbv));
+        const float Hy = __fadd_rn(__fmul_rn(ay, t.y), __fmul_rn(hy[i], t.x));
+        const float Hu = __fadd_rn(__fmul_rn(au, t.y), __fmul_rn(hu[i], t.x));
+        const float Hv = __fadd_rn(__fmul_rn(av, t.y), __fmul_rn(hv[i], t.x));
+        if (pair0(i) < 8) {
+            sy[pair0(i)] = Gy; su[pair0(i)] = Gu; sv[pair0(i)] = Gv;
+            sy[pair1(i)] = Hy; su[pair1(i)] = Hu; sv[pair1(i)] = Hv;
+        } else {
+            oy[pair0(i) - 8] = Gy; ou[pair0(i) - 8] = Gu; ov[pair0(i) - 8] = Gv;
+            oy[pair1(i) - 8] = Hy; ou[pair1(i) - 8] = Hu; ov[pair1(i) - 8] = Hv;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __restrict__ work,
+                                                             const GroupDesc* __restrict__ groups, int ngroups, int parts,
+                                                             const int32_t* __restrict__ items, StateView st,
+                                                             const float* __restrict__ coef,
+                                                             const int32_t* __restrict__ tstatus,
+                                                             const int32_t* __restrict__ rstatus,
+                                                             int32_t* __restrict__ fstatus, OutPtrs o,
+                                                             float* __restrict__ scratch, uint64_t scratch_floats,
+                                                             int* __restrict__ counter) {
+    __shared__ int s_q, s_n, s_intra, s_H, s_ls[kMaxLevels + 1];
+    __shared__ uint32_t s_N, s_lo[kMaxLevels], s_hi[kMaxLevels];  // this part's nodes of each level
+    __shared__ uint64_t s_out[32], s_coef[32];                    // of the slices without an error
+    __shared__ float s_mv[32][12];
+    __shared__ float s_leaf[kFewWarps][3][256];  // a warp's leaves: [yuv][leaf] (also keeps a CTA off a long RLGR CTA's SM)
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    float* const bufA = scratch + (uint64_t)blockIdx.x * scratch_floats;
+    float* const bufB = bufA + scratch_floats / 2;
+    for (;;) {
+        if (tid == 0) s_q = atomicAdd(counter, 1);
+        __syncthreads();
+        const int q = s_q;
+        if (q >= ngroups * parts) break;
+        const GroupDesc G = groups[q / parts];
+        const int part = q % parts;
+        if (tid < 32) {
+            const bool have = tid < G.count;
+            const int item = have ? items[G.first + tid] : 0;
+            const SliceWork& w = work[item];
+            const bool intra_lane = have && G.intra && tid == 0;
+            int err = have ? slice_status(w, item, st, tstatus, rstatus) : PVVC_OK;
+            const int ierr = G.intra ? __shfl_sync(0xffffffffu, err, 0) : PVVC_OK;
+            if (ierr && !intra_lane && have && !err) err = PVVC_ERR_NO_REFERENCE;
+            if (part == 0) {
+                if (ierr && tid == 0) st.info[G.slot].valid = 0;  // a failed intra slice empties the slot
+                if (have) {
+                    fstatus[item] = err;
+                    if (o.status) o.status[w.orig] = err;
+                }
+            }
+            const bool act = have && !err;
+            const uint32_t bal = __ballot_sync(0xffffffffu, act);
+            if (act) {
+                const int f = __popc(bal & ((1u << tid) - 1u));
+                s_out[f] = w.out_off;
+                s_coef[f] = w.coef_off;
+                for (int i = 0; i < 12; ++i) s_mv[f][i] = w.mv[i];
+                s_N = w.n;  // every active slice's: the tree's leaves
+            }
+            if (tid == 0) {
+                s_n = __popc(bal);
+                s_intra = G.intra && !ierr;
+            }
+        } else if (tid == 32) {
+            const SlotInfo* si = st.info + G.slot;
+            s_H = si->height;
+            for (int l = 0; l < kMaxLevels + 1; ++l) s_ls[l] = si->level_start[l];
+        }
+        __syncthreads();
+        const int na = s_n;
+        if (na > 0) {
+            const int H = s_H, fi = s_intra ? 1 : 0;
+            const uint32_t N = s_N;
+            const size_t nb = (size_t)G.slot * st.max_nodes;
+            const size_t lb = (size_t)G.slot * st.max_leaves;
+            if (H == 1) {
+                if (tid == 0 && part == 0)
+                    for (int f = 0; f < na; ++f) {
+                        const float* cy = coef + s_coef[f];
+                        emit_leaf(s_mv[f], s_out[f], N < 10, st, lb, 0, cy[0], cy[N], cy[2ull * N], !(fi && f == 0), o);
+                    }
+            } else {
+                float *gA = bufA, *gB = bufB;
+                const size_t row = 3ull * N;  // a slice's level signal
+                if (tid < na) {
+                    const float* cy = coef + s_coef[tid];
+                    float* g = gA + tid * row;
+                    g[0] = cy[0];
+                    g[1] = cy[N];
+                    g[2] = cy[2ull * N];
+                }
+                if (wid < 2) {
+                    // this part's range of each level, upwards: warp 0 its first
+                    // node, warp 1 its last one (child offsets ascend: a node's
+                    // parent is the last one whose first child is at or below it)
+                    const int cnt = s_ls[H - 1] - s_ls[H - 2], per = (cnt + parts - 1) / parts;
+                    const int j0 = min(cnt, part * per), j1 = min(cnt, j0 + per);
+                    int at = wid == 0 ? j0 : max(j0, j1 - 1);
+                    for (int l = H - 2;; --l) {
+                        if (lane == 0) (wid == 0 ? s_lo : s_hi)[l] = wid == 0 ? at : j0 < j1 ? at + 1 : 0;
+                        if (l == 0) break;
+                        const uint32_t* cb = st.cbase + nb + s_ls[l - 1];
+                        int lo = 0, hi = s_ls[l] - s_ls[l - 1];
+                        while (hi - lo > 1) {
+                            const int step = (hi - lo + 31) >> 5, idx = lo + lane * step;
+                            const uint32_t bal = __ballot_sync(0xffffffffu, idx < hi && (int)__ldg(cb + idx) <= at);
+                            lo += (bal ? 31 - __clz(bal) : 0) * step;
+                            hi = min(hi, lo + step);
+                        }
+                        at = lo;
+                    }
+                }
+                __syncthreads();
+                // this part's nodes of level l of the slices [f0, f0 + nf)
+                auto nodes = [&](int l, int f0, int nf, bool predict) {
+                    const bool last = l == H - 2;
+                    const uint32_t lo = s_lo[l], nj = max(s_hi[l], lo) - lo, nbatch = (nj + 31) / 32;
+                    // the slices in chunks, so that every warp has two units or more
+                    const int chunks = nbatch ? min(nf, (int)((2 * kFewWarps + nbatch - 1) / nbatch)) : 1;
+                    const int per = (nf + chunks - 1) / max(chunks, 1);
+                    for (uint32_t unit = wid; unit < nbatch * chunks; unit += kFewWarps) {
+                        const uint32_t ch = unit / nbatch, j0 = (unit - ch * nbatch) * 32;
+                        const int fa = f0 + (int)ch * per, fb = min(f0 + nf, fa + per);
+                        const uint32_t nv = min(32u, nj - j0), j = lo + j0 + min((uint32_t)lane, nv - 1);
+                        const size_t node = nb + s_ls[l] + j;
+                        LaneNode rec;
+                        rec.byte = (uint32_t)lane < nv ? st.occ[node] : 0u;
+                        rec.m = (uint32_t)lane < nv ? st.mask[node] : 0u;
+                        rec.cb = st.cbase[node];
+                        rec.ci = st.coff[node];
+#pragma unroll
+                        for (int i = 0; i < 7; ++i) rec.ab[i] = __ldg(st.ab + node * 7 + i);
+                        const uint32_t base = __shfl_sync(0xffffffffu, rec.cb, 0);
+                        const uint32_t total = __shfl_sync(0xffffffffu, rec.cb + __popc(rec.byte), nv - 1) - base;
+                        for (int f = fa; f < fb; ++f) {
+                            const float* g = gA + f * row + 3ull * j;
+                            float oy[8], ou[8], ov[8];
+                            lane_inverse(rec, coef + s_coef[f], N, g[0], g[1], g[2], oy, ou, ov);
+                            if (!last) {
+                                float* gb = gB + f * row + 3ull * rec.cb;
+#pragma unroll
+                                for (int c = 0; c < 8; ++c) {
+                                    if (!(rec.byte & (0x80u >> c))) continue;
+                                    gb[0] = oy[c];
+                                    gb[1] = ou[c];
+                                    gb[2] = ov[c];
+                                    gb += 3;
+                                }
+                                continue;
+                            }
+                            float(&lf)[3][256] = s_leaf[wid];
+                            uint32_t at = rec.cb - base;
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) {
+                                if (!(rec.byte & (0x80u >> c))) continue;
+                                lf[0][at] = oy[c];
+                                lf[1][at] = ou[c];
+                                lf[2][at] = ov[c];
+                                ++at;
+                            }
+                            __syncwarp();
+                            const uint64_t out = s_out[f];
+                            for (uint32_t i = lane; i < total; i += 32)
+                                emit_leaf(s_mv[f], out, N < 10, st, lb, base + i, lf[0][i], lf[1][i], lf[2][i], predict, o);
+                            __syncwarp();
+                        }
+                    }
+                };
+                for (int l = 0; l < H - 2; ++l) {
+                    nodes(l, 0, na, true);
+                    __syncthreads();
+                    float* t = gA;
+                    gA = gB;
+                    gB = t;
+                }
+                if (fi) {
+                    nodes(H - 2, 0, 1, false);
+                    __syncthreads();
+                }
+                nodes(H - 2, fi, na - fi, true);
             }
         }
         __syncthreads();
@@ -1638,6 +1876,19 @@ cudaError_t launch_raht_slice(const SliceWork* work, const int32_t* list, int co
     OutPtrs o{xyz, rgb, p24, status};
     k_raht_slice<kRahtThreads><<<count, kRahtThreads, smem, s>>>(work, list, st, coef, fallback, tstatus, rstatus, fstatus, o,
                                                                  wcap);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_raht_few(const SliceWork* work, const GroupDesc* groups, int ngroups, int parts, const int32_t* items,
+                            const StateView& st, const float* coef, const int32_t* tstatus, const int32_t* rstatus,
+                            int32_t* fstatus, float* xyz, uint8_t* rgb, float* p24, int32_t* status, float* scratch,
+                            uint64_t scratch_floats, int nctas, int* counter, cudaStream_t s) {
+    if (ngroups <= 0) return cudaSuccess;
+    if (cudaMemsetAsync(counter, 0, sizeof(int), s) != cudaSuccess) return cudaGetLastError();
+    OutPtrs o{xyz, rgb, p24, status};
+    const int grid = ngroups * parts < nctas ? ngroups * parts : nctas;
+    k_raht_few<<<grid, kFewThreads, 0, s>>>(work, groups, ngroups, parts, items, st, coef, tstatus, rstatus, fstatus, o, scratch,
+                                            scratch_floats, counter);
     return cudaGetLastError();
 }
 

@@ -24,6 +24,10 @@ constexpr int kRlgrLongBlock = 128;
 // the long tier takes kWinGroupsPerLongCta of them per long CTA.
 constexpr int kWinGroupMin = 16;
 constexpr int kWinGroupsPerLongCta = 4;
+// In a batch with window groups, groups of fewer slices (and the long tier's)
+// are inverse-transformed by k_raht_few, the others by k_raht_group; in any other
+// batch all by k_raht_few.
+constexpr int kFewBelow = 16;
 
 struct SliceWork {
     uint64_t col_off;   // colour payload byte offset
@@ -87,11 +91,7 @@ struct GroupDesc {
     int32_t slot;
     int32_t first;  // into the group item list
     int32_t count;  // <= 32
-    int16_t intra;
-    // the inverse transform of a group may be split over `parts` CTAs (0
-    // means 1), each repeating the levels above the last two and taking
-    // part `part` of the last-level nodes
-    uint8_t part, parts;
+    int32_t intra;
 };
 static_assert(sizeof(GroupDesc) == 16, "GroupDesc: four words");
 

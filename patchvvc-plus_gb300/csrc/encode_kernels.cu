@@ -551,6 +551,7 @@ extern "C" int pvvc_encode_colors(pvvc_encoder* enc, const pvvc_batch_desc* desc
     // every slot's slices in groups of up to 32 (no per-slice path), no RLGR split
     const pvvc_tune t{1, 1, 128, -1, -1, 32};
     pvvc_plan& p = enc->plan;
+    p.wide_only = true;
     int rc = build_plan(desc, &p, &t, nullptr);
     if (rc) return rc;
     if (p.max_slot >= st->v.nslots) return PVVC_ERR_ARG;

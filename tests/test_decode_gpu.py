@@ -487,3 +487,55 @@ def test_host_call_zstd_multi_gop_parts(pvvc_lib, torch):
     with pytest.raises(pvvc_lib.PvvcError) as e:
         dec.decode_frames(bad)
     assert e.value.status == 9
+
+
+def _streams(pvvc, frames, streams):
+    """The same GoP `streams` times, in slots of its own: one batch."""
+    one = pvvc.pack_frames([pvvc.parse_frame(b) for b in frames])
+    return one, pvvc.concat_batches([one] * streams, slot_stride=8)
+
+
+# 8 slots: every group a small one, over several CTAs; 160: window groups (as
+# many as an SM each) with a long tier; groups of 1, 2, 15 to 32, and of the 33rd
+# and later frames (without their intra slice)
+@pytest.mark.parametrize("streams,nframes", [(1, 1), (1, 2), (1, 15), (1, 16), (1, 31), (1, 32), (1, 33), (1, 37),
+                                             (20, 15), (20, 17), (20, 37)])
+def test_group_sizes_bit_exact(pvvc_lib, oracle, torch, streams, nframes):
+    frames = _large_value_frames(pvvc_lib, nframes)
+    one, batch = _streams(pvvc_lib, frames, streams)
+    dec = pvvc_lib.Decoder(nslots=8 * streams, max_leaves=4096)
+    xyz, rgb, st, p24 = decode_batch(torch, pvvc_lib, dec, batch, points24=True)
+    assert (st == 0).all(), np.unique(st)
+    P = xyz.shape[0] // streams
+    for s in range(1, streams):
+        for a in (xyz, rgb, p24):
+            assert np.array_equal(a[s * P:(s + 1) * P].view(np.uint8), a[:P].view(np.uint8)), s
+    f = np.float32
+    for fi, (ox, orgb, ost, yuv) in enumerate(oracle_decode(oracle, pvvc_lib, frames, 16)):
+        a, b = one.frame_first_point[fi], one.frame_first_point[fi + 1]
+        assert np.array_equal(xyz[a:b].view(np.uint32), ox.view(np.uint32)), fi
+        y, u, v = yuv[:, 0], yuv[:, 1], yuv[:, 2]
+        want = np.stack([(y + f(1.402) * (v - f(128))) / f(255),
+                         ((y - f(0.3441) * (u - f(128))) - f(0.7141) * (v - f(128))) / f(255),
+                         (y + f(1.772) * (u - f(128))) / f(255)], 1).astype(np.float32)
+        assert np.array_equal(p24[a:b, 3:].view(np.uint32), want.view(np.uint32)), fi
+        assert rgb_matches(rgb[a:b], orgb, yuv).all(), fi
+
+
+@pytest.mark.parametrize("streams,nframes", [(1, 2), (1, 17), (20, 17)])
+def test_failed_intra_fails_its_group_only(pvvc_lib, torch, streams, nframes):
+    """A slot whose intra colours end early: that slice reports the overrun, its
+    other frames no reference, each time; every other slice decodes as before."""
+    parsed = [pvvc_lib.parse_frame(b) for b in _large_value_frames(pvvc_lib, nframes)]
+    good = pvvc_lib.concat_batches([pvvc_lib.pack_frames(parsed)] * streams, slot_stride=8)
+    parsed[0].color[1] = parsed[0].color[1][: len(parsed[0].color[1]) // 4]
+    bad = pvvc_lib.concat_batches([pvvc_lib.pack_frames(parsed)] * streams, slot_stride=8)
+    dec = pvvc_lib.Decoder(nslots=8 * streams, max_leaves=4096)
+    want = decode_batch(torch, pvvc_lib, dec, good)
+    for _ in range(3):
+        xyz, rgb, st = decode_batch(torch, pvvc_lib, dec, bad)
+        hit = bad.slot % 8 == 1
+        assert (st[hit & (bad.type == 1)] == 2).all() and (st[hit & (bad.type == 3)] == 5).all() and (st[~hit] == 0).all()
+        for s in np.flatnonzero(~hit):
+            a, b = int(bad.out_off[s]), int(bad.out_off[s]) + int(bad.size[s])
+            assert np.array_equal(xyz[a:b], want[0][a:b]) and np.array_equal(rgb[a:b], want[1][a:b]), s
