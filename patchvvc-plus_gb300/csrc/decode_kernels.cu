@@ -1776,6 +1776,14 @@ cudaError_t prepare_kernels() {
     std::lock_guard<std::mutex> g(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
     e = cudaFuncSetAttribute(k_raht_slice<kRahtThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    // The tree kernel runs beside the RLGR launches on every SM.  An SM's split of
+    // L1 and shared memory changes only while it is idle: with the tree kernel's
+    // own small share, the RLGR CTAs found room for one or two CTAs on most SMs
+    // and piled up on the others (a medium tier of a 30-frame GoP took 1.43 ms
+    // instead of 0.6; the whole decode 1.98 ms, 1.35 with this).
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_tree<kTreeThreads>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 cudaSharedmemCarveoutMaxShared);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_raht_group<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)sizeof(GroupStage<false>));
