@@ -136,6 +136,8 @@ struct EpiArgs {
     const float* bias;
     const __nv_bfloat16* aux;
     int64_t ldaux;
+    // K block kb's tiles start at (kb * k_step, row + kb * a_step / b_step)
+    int32_t k_step, a_step, b_step;
 };
 
 constexpr int kTileA = kBM * kBK * 2;  // 16 KB
@@ -189,7 +191,8 @@ __device__ __forceinline__ void epilogue_row(uint32_t tl, int row, int M, int n0
                 }
             } else {  // PVVC_GEMM_F32_ACCUM
 #pragma unroll
-                for (int j = 0; j < 32; ++j) atomicAdd(out + j, v[j]);
+                for (int q = 0; q < 8; ++q)
+                    atomicAdd(reinterpret_cast<float4*>(out) + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
             }
         }
     }
@@ -331,8 +334,8 @@ __global__ void __launch_bounds__(kPersistThreads, 1)
                     const uint32_t st = it % S, ph = (it / S) & 1;
                     if (!(ok = mbar_wait(&sm.empty[st], ph ^ 1, 1))) break;
                     mbar_expect_tx(&sm.full[st], (kBM + BN) * kBK * 2);
-                    tma_load_2d(tile_a(st), &map_a, &sm.full[st], kb * kBK, m0);
-                    tma_load_2d(tile_b(st), &map_b, &sm.full[st], kb * kBK, n0);
+                    tma_load_2d(tile_a(st), &map_a, &sm.full[st], kb * ep.k_step, m0 + kb * ep.a_step);
+                    tma_load_2d(tile_b(st), &map_b, &sm.full[st], kb * ep.k_step, n0 + kb * ep.b_step);
                 }
             }
         }
@@ -481,11 +484,25 @@ int gemm_bf16(int32_t M, int32_t N, int32_t K, const void* A, int64_t lda, const
     const int BN = N % 256 == 0 ? 256 : N % 128 == 0 ? 128 : 64;
     CUtensorMap ma, mb;
     if (!make_map(&ma, A, M, K, lda, kBM) || !make_map(&mb, B, N, K, ldb, BN)) return PVVC_ERR_CUDA;
-    EpiArgs ep{C, ldc, bias, static_cast<const __nv_bfloat16*>(aux), ldaux};
+    EpiArgs ep{C, ldc, bias, static_cast<const __nv_bfloat16*>(aux), ldaux, kBK, 0, 0};
     cudaError_t e = BN == 256 ? launch_epi<256>(epi, ma, mb, M, N, K, splits, ep, s)
                   : BN == 128 ? launch_epi<128>(epi, ma, mb, M, N, K, splits, ep, s)
                               : launch_epi<64>(epi, ma, mb, M, N, K, splits, ep, s);
     return e == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;
+}
+
+// C[128, 64] += A B^T over K = 64 * nkb, split over `splits`, with the operands in
+// blocks of 64 of K: A[kb][128][64], B[kb][64][64].  A block is one contiguous run,
+// for the kernels that write it as for its TMA loads.  K = 524,288: 68 us over two
+// splits an SM, each adding its 8,192 sums one by one; 39 with one split an SM
+// adding four at a time (201 MB read).
+int gemm_bf16_blocked(int32_t nkb, const void* A, const void* B, float* C, int64_t ldc, int32_t splits, cudaStream_t s) {
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, A, (int64_t)nkb * 128, kBK, kBK, kBM) || !make_map(&mb, B, (int64_t)nkb * 64, kBK, kBK, 64))
+        return PVVC_ERR_CUDA;
+    EpiArgs ep{C, ldc, nullptr, nullptr, 0, 0, 128, 64};
+    return launch_epi<64>(PVVC_GEMM_F32_ACCUM, ma, mb, 128, 64, nkb * kBK, splits, ep, s) == cudaSuccess ? PVVC_OK
+                                                                                                        : PVVC_ERR_CUDA;
 }
 
 int device_error_take(int* code) {

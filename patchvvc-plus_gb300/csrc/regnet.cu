@@ -39,6 +39,7 @@ namespace pvvc {
 int gemm_bf16(int32_t M, int32_t N, int32_t K, const void* A, int64_t lda, const void* B, int64_t ldb, void* C,
               int64_t ldc, const float* bias, const void* aux, int64_t ldaux, int32_t epi, int32_t splits,
               cudaStream_t s);
+int gemm_bf16_blocked(int32_t nkb, const void* A, const void* B, float* C, int64_t ldc, int32_t splits, cudaStream_t s);
 
 namespace {
 
@@ -92,9 +93,10 @@ __device__ __forceinline__ float block_sum256(float v, float* red) {
     return t;
 }
 
-// X1 row = relu(W1 x0 + b1) as 64 bf16 (128 bytes)
+// X1 row = relu(W1 x0 + b1) as 64 bf16 (128 bytes); with `outT`, also into the
+// transpose (blocks of [channel][64 rows]; channel c at outT[64 c])
 __device__ __forceinline__ void layer1_row(const float* w1, const float* b1, float x, float y, float z,
-                                           __nv_bfloat16* out) {
+                                           __nv_bfloat16* out, __nv_bfloat16* outT) {
     uint4* o4 = reinterpret_cast<uint4*>(out);
 #pragma unroll
     for (int q = 0; q < kD1 / 8; ++q) {
@@ -111,6 +113,10 @@ __device__ __forceinline__ void layer1_row(const float* w1, const float* b1, flo
                                            b1[b]),
                                    0.f);
             h[j] = __floats2bfloat162_rn(va, vb);
+            if (outT) {
+                outT[64 * a] = h[j].x;
+                outT[64 * b] = h[j].y;
+            }
         }
         o4[q] = *reinterpret_cast<uint4*>(h);
     }
@@ -126,7 +132,7 @@ __global__ void __launch_bounds__(256) k_sample_l1(int npairs, const int32_t* __
                                                    const uint32_t* __restrict__ toff, uint64_t seed,
                                                    const float* __restrict__ w1, const float* __restrict__ b1,
                                                    float* __restrict__ x0, __nv_bfloat16* __restrict__ x1,
-                                                   float* __restrict__ frame, const float* __restrict__ T_label,
+                                                   __nv_bfloat16* __restrict__ x1t, float* __restrict__ frame, const float* __restrict__ T_label,
                                                    const float* __restrict__ omega_label, float* __restrict__ y) {
     __shared__ float red[8];
     const int b = blockIdx.x, j = threadIdx.x;
@@ -153,7 +159,7 @@ __global__ void __launch_bounds__(256) k_sample_l1(int npairs, const int32_t* __
         x0[3 * row] = x;
         x0[3 * row + 1] = yy;
         x0[3 * row + 2] = z;
-        layer1_row(w1, b1, x, yy, z, x1 + row * kD1);
+        layer1_row(w1, b1, x, yy, z, x1 + row * kD1, x1t ? x1t + (row / 64 * kD1) * 64 + row % 64 : nullptr);
     }
     if (j == 0) {
         float* f = frame + 7 * b;
@@ -173,12 +179,44 @@ __global__ void __launch_bounds__(256) k_sample_l1(int npairs, const int32_t* __
     }
 }
 
-// X1 from given x0 rows (the gradient-check entry)
-__global__ void k_l1(int64_t rows, const float* __restrict__ x0, const float* __restrict__ w1, const float* __restrict__ b1,
-                     __nv_bfloat16* __restrict__ x1) {
-    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= rows) return;
-    layer1_row(w1, b1, x0[3 * r], x0[3 * r + 1], x0[3 * r + 2], x1 + r * kD1);
+// X1 and its transpose from given x0 rows (the gradient-check entry), 256 rows a
+// block, both written in whole lines through shared memory: layer 2's weight
+// gradient reads the transpose (blocks of [channel][64 rows]).  For 524,288 rows 41 us with a row a thread and
+// 42 more for a transpose kernel; 25 now (134 MB written).
+constexpr int kL1Row = kD1 / 2 + 1;  // words of a staged row: odd, so that a column's words spread over the banks
+__global__ void __launch_bounds__(256) k_l1(int64_t rows, const float* __restrict__ x0, const float* __restrict__ w1,
+                                            const float* __restrict__ b1, __nv_bfloat16* __restrict__ x1,
+                                            __nv_bfloat16* __restrict__ x1t) {
+    __shared__ float4 s_w[kD1];
+    __shared__ uint32_t s_t[256 * kL1Row];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int64_t r0 = blockIdx.x * 256ll;  // rows is a multiple of 256
+    if (t < kD1) s_w[t] = make_float4(w1[3 * t], w1[3 * t + 1], w1[3 * t + 2], b1[t]);
+    const float x = x0[3 * (r0 + t)], y = x0[3 * (r0 + t) + 1], z = x0[3 * (r0 + t) + 2];
+    __syncthreads();
+    auto channel = [&](int c) {
+        const float4 w = s_w[c];
+        return fmaxf(__fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(w.x, x), __fmul_rn(w.y, y)), __fmul_rn(w.z, z)), w.w), 0.f);
+    };
+#pragma unroll 8
+    for (int c = 0; c < kD1; c += 2) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(channel(c), channel(c + 1));
+        s_t[t * kL1Row + c / 2] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    __syncthreads();
+    uint32_t* o = reinterpret_cast<uint32_t*>(x1 + r0 * kD1);
+#pragma unroll 8
+    for (int i = t; i < 256 * kD1 / 2; i += 256) o[i] = s_t[(i / (kD1 / 2)) * kL1Row + i % (kD1 / 2)];
+    // channel pair wid + 8 i, rows 2 lane and 2 lane + 1 of each 64
+    for (int cp = wid; cp < kD1 / 2; cp += 8)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int row = 64 * q + 2 * lane;
+            const uint32_t u = s_t[row * kL1Row + cp], v = s_t[(row + 1) * kL1Row + cp];
+            uint32_t* o = reinterpret_cast<uint32_t*>(x1t + ((r0 / 64 + q) * kD1 + 2 * cp) * 64) + lane;
+            o[0] = __byte_perm(u, v, 0x5410);
+            o[32] = __byte_perm(u, v, 0x7632);
+        }
 }
 
 // max over each cloud's P rows of Y3 (first maximum), into H0 = [G_src | G_tgt]
@@ -254,37 +292,19 @@ __global__ void k_transpose(const __nv_bfloat16* __restrict__ in, int64_t R, int
 
 // out[C,R] = in[R,C]^T for even R and C: 64x64 tiles, each thread moving
 // bf16 pairs, so that a warp reads and writes 128 contiguous bytes per row.
-// part (optional): the tile's column sums, part[blockIdx.y * C + c], for
-// k_colsum_parts.
 __global__ void __launch_bounds__(256) k_transpose_pairs(const __nv_bfloat16* __restrict__ in, int64_t R, int64_t C,
-                                                         __nv_bfloat16* __restrict__ out, float* __restrict__ part) {
+                                                         __nv_bfloat16* __restrict__ out) {
     __shared__ __nv_bfloat16 t[64][66];  // odd word stride: column reads spread over the banks
-    __shared__ float red[8][64];
     const int64_t r0 = blockIdx.y * 64ll, c0 = blockIdx.x * 64ll;
     const int tx = threadIdx.x, ty = threadIdx.y;
-    float s0 = 0.f, s1 = 0.f;
     for (int i = ty; i < 64; i += 8) {
         const int64_t r = r0 + i, c = c0 + 2 * tx;
         __nv_bfloat162 v = __floats2bfloat162_rn(0.f, 0.f);
         if (r < R && c < C) v = *reinterpret_cast<const __nv_bfloat162*>(in + r * C + c);
         t[i][2 * tx] = v.x;
         t[i][2 * tx + 1] = v.y;
-        s0 += __bfloat162float(v.x);
-        s1 += __bfloat162float(v.y);
-    }
-    if (part) {
-        red[ty][2 * tx] = s0;
-        red[ty][2 * tx + 1] = s1;
     }
     __syncthreads();
-    if (part && ty == 0) {
-        for (int h = 0; h < 2; ++h) {
-            const int64_t c = c0 + 2 * tx + h;
-            float a = 0.f;
-            for (int y = 0; y < 8; ++y) a += red[y][2 * tx + h];
-            if (c < C) part[blockIdx.y * C + c] = a;
-        }
-    }
     for (int i = ty; i < 64; i += 8) {
         const int64_t c = c0 + i, r = r0 + 2 * tx;
         if (c < C && r < R) {
@@ -391,96 +411,180 @@ __global__ void __launch_bounds__(kD2) k_pool_bwd_w3(int nclouds, const float* _
 // channels with a gradient are bucketed by their argmax row (a stable
 // counting sort: channel order kept within a row); then each row's 128
 // outputs are summed over its bucket in channel order and written at once,
-// zero rows included, as column pairs (four rows per pass).
-__global__ void __launch_bounds__(256) k_pool_bwd_x2(const float* __restrict__ dh0, const __nv_bfloat16* __restrict__ h0,
+// zero rows included: a warp takes 16 rows of each half, a lane four columns,
+// eight rows' X2 in flight.  The block also writes its part of dY2's transpose
+// (dY2T, blocks of [channel][64 rows], for the weight gradient) and its column sums (for db2) from the rows in shared memory,
+// instead of kernels that read dY2 again: 1,024 pairs took 117 us and 85 more for
+// the transpose; 113 now (402 MB read and written).
+constexpr int kDyRow = kD2 + 2;  // staged row of dY2 (bf16): 65 words, odd
+__global__ void __launch_bounds__(256, 4) k_pool_bwd_x2(const float* __restrict__ dh0, const __nv_bfloat16* __restrict__ h0,
                                                     const int32_t* __restrict__ amax, const __nv_bfloat16* __restrict__ w3,
-                                                    const __nv_bfloat16* __restrict__ x2, __nv_bfloat16* __restrict__ dy2) {
-    static_assert(kD3 == 256 && kP == 256 && kD2 == 128, "one thread per channel and per row; 64 column pairs x 4 rows per pass");
+                                                    const __nv_bfloat16* __restrict__ x2, __nv_bfloat16* __restrict__ dy2,
+                                                    __nv_bfloat16* __restrict__ dy2t, float* __restrict__ part) {
+    static_assert(kD3 == 256 && kP == 256 && kD2 == 128, "one thread per channel and per row; 32 lanes x 4 columns");
+    __shared__ uint32_t s_dy[kP / 2 * kDyRow / 2];  // half the rows, [kDyRow] bf16 each
     __shared__ float s_g[kD3];
     __shared__ int32_t s_row[kD3];
     __shared__ int32_t s_start[kP + 1];  // bucket of row r: s_list[s_start[r] .. s_start[r + 1])
-    __shared__ int32_t s_list[kD3];
-    const int c = blockIdx.x, t = threadIdx.x;
+    __shared__ int32_t s_list[kD3], s_any[kD3], s_fill[kP];
+    __shared__ int32_t s_warp[8];
+    __shared__ float s_sum[8][kD2];
+    const int c = blockIdx.x, t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    const int64_t base = (int64_t)c * kP;
     const float g = pooled_grad(dh0, h0, c, t);
     const int r = amax[c * kD3 + t];
     s_g[t] = g;
     s_row[t] = g != 0.f ? r : -1;
+    s_start[t] = 0;
     __syncthreads();
-    // count of row t (thread t), then an exclusive scan over the 256 rows
-    int cnt = 0;
-    for (int n = 0; n < kD3; ++n) cnt += s_row[n] == t;
+    // channels with a gradient bucketed by row: counts, an exclusive scan, slots in
+    // any order, then each channel's place among its row's (channel order)
+    if (s_row[t] >= 0) atomicAdd(&s_start[s_row[t]], 1);
+    __syncthreads();
+    const int cnt = s_start[t];
     int x = cnt;
-    const int lane = t & 31, wid = t >> 5;
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    __shared__ int32_t s_warp[8];
     if (lane == 31) s_warp[wid] = x;
     __syncthreads();
     int before = 0;
     for (int w = 0; w < wid; ++w) before += s_warp[w];
-    s_start[t] = before + x - cnt;
-    if (t == kP - 1) s_start[kP] = before + x;
+    const int end = before + x;
+    s_start[t] = end - cnt;
+    s_fill[t] = end - cnt;
+    if (t == kP - 1) s_start[kP] = end;
     __syncthreads();
-    // channel t goes after the channels below it with the same row
+    if (s_row[t] >= 0) s_any[atomicAdd(&s_fill[s_row[t]], 1)] = t;
+    __syncthreads();
     if (s_row[t] >= 0) {
+        const int b0 = s_start[s_row[t]], b1 = s_start[s_row[t] + 1];
         int rank = 0;
-        for (int n = 0; n < t; ++n) rank += s_row[n] == s_row[t];
-        s_list[s_start[s_row[t]] + rank] = t;
+        for (int j = b0; j < b1; ++j) rank += s_any[j] < t;
+        s_list[b0 + rank] = t;
     }
     __syncthreads();
-    // column pair kp of rows r0 + quarter: a warp moves 128 contiguous bytes
-    const int kp = t & (kD2 / 2 - 1), quarter = t >> 6;
-    const int64_t base = (int64_t)c * kP;
-    for (int r0 = 0; r0 < kP; r0 += 4) {
-        const int row = r0 + quarter;
-        float a0 = 0.f, a1 = 0.f;
-        for (int j = s_start[row]; j < s_start[row + 1]; ++j) {
-            const int n = s_list[j];
-            const __nv_bfloat162 w = *reinterpret_cast<const __nv_bfloat162*>(w3 + n * kD2 + 2 * kp);
-            a0 += s_g[n] * __bfloat162float(w.x);
-            a1 += s_g[n] * __bfloat162float(w.y);
+    const uint2* xr = reinterpret_cast<const uint2*>(x2 + base * kD2) + lane;  // row's columns 4 lane ..
+    uint2* dr = reinterpret_cast<uint2*>(dy2 + base * kD2) + lane;
+    const uint2* wr = reinterpret_cast<const uint2*>(w3) + lane;
+    float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    auto lo = [](uint32_t u) { return __uint_as_float(u << 16); };
+    auto hi = [](uint32_t u) { return __uint_as_float(u & 0xFFFF0000u); };
+    for (int half = 0; half < 2; ++half) {
+        for (int i0 = 0; i0 < 16; i0 += 8) {
+            const int first = 128 * half + 16 * wid + i0;
+            uint2 xv[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) xv[i] = __ldg(xr + (first + i) * (kD2 / 4));
+            // each row's first channel (most have at most one), eight loads in flight
+            int at[9];
+            uint2 w0[8];
+            float g0[8];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) at[i] = s_start[first + i];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const bool some = at[i] < at[i + 1];
+                const int n = some ? s_list[at[i]] : 0;
+                w0[i] = some ? __ldg(wr + n * (kD2 / 4)) : make_uint2(0u, 0u);
+                g0[i] = some ? s_g[n] : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int row = first + i, srow = row & 127;
+                float a[4] = {0.f, 0.f, 0.f, 0.f};
+                auto add = [&](float gn, const uint2& w) {
+                    a[0] += gn * lo(w.x);
+                    a[1] += gn * hi(w.x);
+                    a[2] += gn * lo(w.y);
+                    a[3] += gn * hi(w.y);
+                };
+                if (at[i] < at[i + 1]) add(g0[i], w0[i]);
+                for (int j = at[i] + 1; j < at[i + 1]; ++j) {
+                    const int n = s_list[j];
+                    add(s_g[n], __ldg(wr + n * (kD2 / 4)));
+                }
+                const __nv_bfloat162 p = __floats2bfloat162_rn(lo(xv[i].x) > 0.f ? a[0] : 0.f, hi(xv[i].x) > 0.f ? a[1] : 0.f);
+                const __nv_bfloat162 q = __floats2bfloat162_rn(lo(xv[i].y) > 0.f ? a[2] : 0.f, hi(xv[i].y) > 0.f ? a[3] : 0.f);
+                const uint2 d = make_uint2(*reinterpret_cast<const uint32_t*>(&p), *reinterpret_cast<const uint32_t*>(&q));
+                dr[row * (kD2 / 4)] = d;
+                s_dy[srow * (kDyRow / 2) + 2 * lane] = d.x;
+                s_dy[srow * (kDyRow / 2) + 2 * lane + 1] = d.y;
+                sum[0] += lo(d.x);
+                sum[1] += hi(d.x);
+                sum[2] += lo(d.y);
+                sum[3] += hi(d.y);
+            }
         }
-        const int64_t idx = (base + row) * kD2 + 2 * kp;
-        const __nv_bfloat162 xv = *reinterpret_cast<const __nv_bfloat162*>(x2 + idx);
-        *reinterpret_cast<__nv_bfloat162*>(dy2 + idx) = __floats2bfloat162_rn(__bfloat162float(xv.x) > 0.f ? a0 : 0.f,
-                                                                               __bfloat162float(xv.y) > 0.f ? a1 : 0.f);
+        __syncthreads();
+        // column pair cp, rows 2 lane and 2 lane + 1 of each 64
+        for (int cp = wid; cp < kD2 / 2; cp += 8)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int row = 64 * q + 2 * lane;
+                const uint32_t u = s_dy[row * (kDyRow / 2) + cp], v = s_dy[(row + 1) * (kDyRow / 2) + cp];
+                uint32_t* o = reinterpret_cast<uint32_t*>(dy2t + ((base / 64 + 2 * half + q) * kD2 + 2 * cp) * 64) + lane;
+                o[0] = __byte_perm(u, v, 0x5410);
+                o[32] = __byte_perm(u, v, 0x7632);
+            }
+        __syncthreads();
+    }
+    for (int i = 0; i < 4; ++i) s_sum[wid][4 * lane + i] = sum[i];
+    __syncthreads();
+    if (t < kD2) {
+        float a = 0.f;
+        for (int w = 0; w < 8; ++w) a += s_sum[w][t];
+        part[(int64_t)c * kD2 + t] = a;
     }
 }
 
-// dW1 += dY1^T x0, db1 += colsum(dY1): 64 outputs x 4 row phases per block
+// dW1 += dY1^T x0, db1 += colsum(dY1).  A lane takes 8 of a row's 64 outputs (a
+// warp four rows a load, four loads in flight); the blocks, a few per SM, combine
+// by atomics.  524,288 rows: 61 us with an output a thread, 28 now (73 MB read).
 __global__ void __launch_bounds__(256) k_bwd_w1(const __nv_bfloat16* __restrict__ dy1, const float* __restrict__ x0, int64_t R,
                                                int64_t rows_per_block, float* __restrict__ gw1, float* __restrict__ gb1) {
-    __shared__ float red[4][kD1][4];
-    const int o = threadIdx.x & 63, ph = threadIdx.x >> 6;
+    __shared__ float red[8][4][kD1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = lane & 7, sub = lane >> 3;
     const int64_t r0 = blockIdx.x * rows_per_block, r1 = min(R, r0 + rows_per_block);
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, ab = 0.f;
-#pragma unroll 4
-    for (int64_t r = r0 + ph; r < r1; r += 4) {
-        const float d = __bfloat162float(dy1[r * kD1 + o]);
-        a0 += d * x0[3 * r];
-        a1 += d * x0[3 * r + 1];
-        a2 += d * x0[3 * r + 2];
-        ab += d;
-    }
-    red[ph][o][0] = a0;
-    red[ph][o][1] = a1;
-    red[ph][o][2] = a2;
-    red[ph][o][3] = ab;
-    __syncthreads();
-    if (ph == 0) {
-        for (int q = 1; q < 4; ++q) {
-            a0 += red[q][o][0];
-            a1 += red[q][o][1];
-            a2 += red[q][o][2];
-            ab += red[q][o][3];
+    float a[8][4] = {};
+    for (int64_t r = r0 + 4 * wid + sub; r < r1; r += 128) {
+        uint4 d[4];
+        float x[4][3];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t row = r + 32 * u;
+            const bool in = row < r1;
+            d[u] = in ? __ldg(reinterpret_cast<const uint4*>(dy1 + row * kD1) + q) : make_uint4(0u, 0u, 0u, 0u);
+            for (int k = 0; k < 3; ++k) x[u][k] = in ? __ldg(x0 + 3 * row + k) : 0.f;
         }
-        atomicAdd(gw1 + 3 * o, a0);
-        atomicAdd(gw1 + 3 * o + 1, a1);
-        atomicAdd(gw1 + 3 * o + 2, a2);
-        atomicAdd(gb1 + o, ab);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t w[4] = {d[u].x, d[u].y, d[u].z, d[u].w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float v = __uint_as_float(j & 1 ? w[j / 2] & 0xFFFF0000u : w[j / 2] << 16);
+                a[j][0] += v * x[u][0];
+                a[j][1] += v * x[u][1];
+                a[j][2] += v * x[u][2];
+                a[j][3] += v;
+            }
+        }
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float v = a[j][k];
+            v += __shfl_xor_sync(0xffffffffu, v, 8);
+            v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (sub == 0) red[wid][k][8 * q + j] = v;
+        }
+    __syncthreads();
+    const int o = threadIdx.x & 63, k = threadIdx.x >> 6;
+    float v = 0.f;
+    for (int w = 0; w < 8; ++w) v += red[w][k][o];
+    atomicAdd(k < 3 ? gw1 + 3 * o + k : gb1 + o, v);
 }
 
 // AdamW on the flat fp32 vector (decoupled weight decay on weight matrices only)
@@ -554,8 +658,11 @@ struct pvvc_regnet {
     int64_t step = 0;
     // activations and scratch for up to `cap` pairs
     int64_t cap = 0;
-    DevBuf x0, x1, x2, y3, h0, amax, h1, h2, out, frame, y, dh2, dh1, dh0, dy2, dy1, ta, tb, loss, ids;
-    DevBuf part;  // column sums of dY2 per 64-row tile (the db2 reduction)
+    DevBuf x0, x1, x2, y3, h0, amax, h1, h2, out, frame, y, dh2, dh1, dh0, dy2, dy1, loss, ids;
+    DevBuf x1t, dy2t;  // transposes (the weight gradient of layer 2)
+    DevBuf ta, tb;     // ... of the head layers' operands
+    SideStream side;   // the weight gradients that nothing else of the pass waits for
+    DevBuf part;       // column sums of dY2 per cloud (the db2 reduction)
 };
 
 namespace {
@@ -577,10 +684,11 @@ int ensure_cap(pvvc_regnet* n, int64_t B) {
               n->y.ensure(4 * B * kOut) == cudaSuccess && n->dh2.ensure(2 * B * kH2) == cudaSuccess &&
               n->dh1.ensure(2 * B * kH1) == cudaSuccess && n->dh0.ensure(4 * B * kH0) == cudaSuccess &&
               n->dy2.ensure(2 * M * kD2) == cudaSuccess && n->dy1.ensure(2 * M * kD1) == cudaSuccess &&
-              n->ta.ensure(2 * M * kD2) == cudaSuccess && n->tb.ensure(2 * M * kD1 + 2 * B * kH0) == cudaSuccess &&
+              n->dy2t.ensure(2 * M * kD2) == cudaSuccess && n->x1t.ensure(2 * M * kD1) == cudaSuccess &&
+              n->ta.ensure(2 * B * std::max(kH1, kH2)) == cudaSuccess && n->tb.ensure(2 * B * std::max(kH0, kH1)) == cudaSuccess &&
               n->loss.ensure(16) == cudaSuccess && n->ids.ensure(4 * B) == cudaSuccess &&
-              n->part.ensure(4 * ((M + 63) / 64) * kD2) == cudaSuccess;
-    if (!ok) return PVVC_ERR_NOMEM;
+              n->part.ensure(4 * 2 * B * kD2) == cudaSuccess;
+    if (!ok || n->side.ensure() != cudaSuccess) return PVVC_ERR_NOMEM;
     n->cap = B;
     return PVVC_OK;
 }
@@ -631,28 +739,18 @@ int forward_from_x1(pvvc_regnet* n, int64_t B, const float* y, float lambda_w, b
 }
 
 // dW += dY^T X over `rows` rows: transposes into scratch, then a split-K GEMM.
-// With gb and part (scratch of ceil(rows/64) * dout floats) and even sizes,
-// the transpose of dY also yields db += column sums of dY.
 int weight_grad(int64_t rows, int dout, int din, const __nv_bfloat16* dy, const __nv_bfloat16* x, __nv_bfloat16* dyT,
-                __nv_bfloat16* xT, float* gw, cudaStream_t s, float* gb = nullptr, float* part = nullptr) {
+                __nv_bfloat16* xT, float* gw, cudaStream_t s) {
     const bool pairs = rows % 2 == 0 && dout % 2 == 0 && din % 2 == 0;
-    auto transpose = [&](const __nv_bfloat16* in, int cols, __nv_bfloat16* out, float* prt) {
+    auto transpose = [&](const __nv_bfloat16* in, int cols, __nv_bfloat16* out) {
         dim3 blk(32, 8);
         if (pairs)
-            k_transpose_pairs<<<dim3((cols + 63) / 64, (unsigned)((rows + 63) / 64)), blk, 0, s>>>(in, rows, cols, out, prt);
+            k_transpose_pairs<<<dim3((cols + 63) / 64, (unsigned)((rows + 63) / 64)), blk, 0, s>>>(in, rows, cols, out);
         else
             k_transpose<<<dim3((cols + 31) / 32, (unsigned)((rows + 31) / 32)), blk, 0, s>>>(in, rows, cols, out);
     };
-    const bool fused_db = gb && part && pairs;
-    transpose(dy, dout, dyT, fused_db ? part : nullptr);
-    if (fused_db) {
-        const int64_t nparts = (rows + 63) / 64, per = 128;
-        k_colsum_parts<<<dim3((dout + 31) / 32, (unsigned)((nparts + per - 1) / per)), dim3(32, 8), 0, s>>>(part, nparts, dout,
-                                                                                                         per, gb);
-    } else if (gb) {
-        k_colsum<<<(unsigned)((rows + 1023) / 1024), 128, 0, s>>>(dy, rows, dout, 1024, gb);
-    }
-    transpose(x, din, xT, nullptr);
+    transpose(dy, dout, dyT);
+    transpose(x, din, xT);
     const int nkb = (int)(rows / 64);
     const int splits = std::max(1, std::min(nkb, 2 * sm_count() / std::max(1, (dout + 127) / 128)));
     return gemm_bf16(dout, din, (int32_t)rows, dyT, rows, xT, rows, gw, din, nullptr, nullptr, 0, PVVC_GEMM_F32_ACCUM,
@@ -664,31 +762,37 @@ int backward(pvvc_regnet* n, int64_t B, cudaStream_t s) {
     const int64_t M = 2 * B * kP;
     float* g = F32(g);
     int rc;
-    // head layers: dW5, db5, dH1
-    if ((rc = weight_grad(B, kH2, kH1, BF(dh2), BF(h1), BF(ta), BF(tb), g + kL.w5, s))) return rc;
-    k_colsum<<<(unsigned)((B + 63) / 64), 128, 0, s>>>(BF(dh2), B, kH2, 64, g + kL.b5);
+    // The chain dH1, dH0, dY2, dY1 on this stream; the weight gradients of the head
+    // layers (small kernels, 100 us of launches one after another) and of layer 3
+    // (gathers, bound by latency) beside it on the side stream.
+    const SideStream& w = n->side;
     if ((rc = gemm_bf16((int32_t)B, kH1, kH2, BF(dh2), kH2, BF(w5t), kH2, BF(dh1), kH1, nullptr, BF(h1), kH1,
                         PVVC_GEMM_MASK_BF16, 1, s)))
         return rc;
-    // dW4, db4, dH0 (fp32)
-    if ((rc = weight_grad(B, kH1, kH0, BF(dh1), BF(h0), BF(ta), BF(tb), g + kL.w4, s))) return rc;
-    k_colsum<<<(unsigned)((B + 63) / 64), 256, 0, s>>>(BF(dh1), B, kH1, 64, g + kL.b4);
     if ((rc = gemm_bf16((int32_t)B, kH0, kH1, BF(dh1), kH1, BF(w4t), kH1, F32(dh0), kH0, nullptr, nullptr, 0, PVVC_GEMM_F32,
                         1, s)))
         return rc;
-    // max-pool + layer 3 (sparse): dW3, db3, dY2
-    k_pool_bwd_w3<<<dim3(kD3, kPoolParts), kD2, 0, s>>>((int)(2 * B), F32(dh0), BF(h0), static_cast<int32_t*>(n->amax.p), BF(x2), g + kL.w3,
-                                      g + kL.b3);
-    k_pool_bwd_x2<<<(unsigned)(2 * B), 256, 0, s>>>(F32(dh0), BF(h0), static_cast<int32_t*>(n->amax.p),
-                                                                            BF(w3b), BF(x2), BF(dy2));
-    // layer 2: dW2, db2, dY1
-    if ((rc = weight_grad(M, kD2, kD1, BF(dy2), BF(x1), BF(ta), BF(tb), g + kL.w2, s, g + kL.b2, F32(part))))
-        return rc;
+    if (cudaEventRecord(w.fork, s) != cudaSuccess || cudaStreamWaitEvent(w.s, w.fork, 0) != cudaSuccess) return PVVC_ERR_CUDA;
+    // dW3, db3; dW4, db4; dW5, db5
+    k_pool_bwd_w3<<<dim3(kD3, kPoolParts), kD2, 0, w.s>>>((int)(2 * B), F32(dh0), BF(h0), static_cast<int32_t*>(n->amax.p),
+                                                          BF(x2), g + kL.w3, g + kL.b3);
+    if ((rc = weight_grad(B, kH1, kH0, BF(dh1), BF(h0), BF(ta), BF(tb), g + kL.w4, w.s))) return rc;
+    k_colsum<<<(unsigned)((B + 63) / 64), 256, 0, w.s>>>(BF(dh1), B, kH1, 64, g + kL.b4);
+    if ((rc = weight_grad(B, kH2, kH1, BF(dh2), BF(h1), BF(ta), BF(tb), g + kL.w5, w.s))) return rc;
+    k_colsum<<<(unsigned)((B + 63) / 64), 128, 0, w.s>>>(BF(dh2), B, kH2, 64, g + kL.b5);
+    // max-pool + layer 3 (sparse): dY2
+    k_pool_bwd_x2<<<(unsigned)(2 * B), 256, 0, s>>>(F32(dh0), BF(h0), static_cast<int32_t*>(n->amax.p), BF(w3b),
+                                                               BF(x2), BF(dy2), BF(dy2t), F32(part));
+    // layer 2: dW2 (x1t: written with X1), db2, dY1
+    k_colsum_parts<<<dim3(kD2 / 32, (unsigned)((2 * B + 63) / 64)), dim3(32, 8), 0, s>>>(F32(part), 2 * B, kD2, 64, g + kL.b2);
+    if ((rc = gemm_bf16_blocked((int32_t)(M / 64), BF(dy2t), BF(x1t), g + kL.w2, kD1, sm_count(), s))) return rc;
     if ((rc = gemm_bf16((int32_t)M, kD1, kD2, BF(dy2), kD2, BF(w2t), kD2, BF(dy1), kD1, nullptr, BF(x1), kD1,
                         PVVC_GEMM_MASK_BF16, 1, s)))
         return rc;
     // layer 1
-    k_bwd_w1<<<(unsigned)((M + 511) / 512), 256, 0, s>>>(BF(dy1), F32(x0), M, 512, g + kL.w1, g + kL.b1);
+    const int64_t per = std::max<int64_t>(512, (M + 4 * sm_count() - 1) / (4 * sm_count()));
+    k_bwd_w1<<<(unsigned)((M + per - 1) / per), 256, 0, s>>>(BF(dy1), F32(x0), M, per, g + kL.w1, g + kL.b1);
+    if (cudaEventRecord(w.join, w.s) != cudaSuccess || cudaStreamWaitEvent(s, w.join, 0) != cudaSuccess) return PVVC_ERR_CUDA;
     return cudaGetLastError() == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;
 }
 
@@ -768,7 +872,7 @@ extern "C" int pvvc_regnet_grad(pvvc_regnet* n, int32_t npairs, const float* x0,
         cudaMemsetAsync(n->g.p, 0, 4ull * n->nparam, s) != cudaSuccess || cudaMemsetAsync(n->loss.p, 0, 4, s) != cudaSuccess)
         return PVVC_ERR_CUDA;
     const float* p = F32(p);
-    k_l1<<<(unsigned)((M + 255) / 256), 256, 0, s>>>(M, F32(x0), p + kL.w1, p + kL.b1, BF(x1));
+    k_l1<<<(unsigned)(M / 256), 256, 0, s>>>(M, F32(x0), p + kL.w1, p + kL.b1, BF(x1), BF(x1t));
     if ((rc = forward_from_x1(n, B, F32(y), lambda_w, true, s))) return rc;
     if ((rc = backward(n, B, s))) return rc;
     if (grad_out && cudaMemcpyAsync(grad_out, n->g.p, 4ull * n->nparam, cudaMemcpyDeviceToDevice, s) != cudaSuccess)
@@ -792,7 +896,7 @@ extern "C" int pvvc_regnet_train_step(pvvc_regnet* n, int32_t npairs, const int3
         return PVVC_ERR_CUDA;
     const float* p = F32(p);
     k_sample_l1<<<(unsigned)B, kP, 0, s>>>((int)B, pair_ids, src, src_off, tgt, tgt_off, seed, p + kL.w1, p + kL.b1, F32(x0),
-                                           BF(x1), F32(frame), T_label, omega_label, F32(y));
+                                           BF(x1), BF(x1t), F32(frame), T_label, omega_label, F32(y));
     if ((rc = forward_from_x1(n, B, F32(y), opt->lambda_w, true, s))) return rc;
     if ((rc = backward(n, B, s))) return rc;
     n->step++;
@@ -817,7 +921,7 @@ extern "C" int pvvc_propose(pvvc_regnet* n, int32_t npairs, const float* src, co
     const int64_t B = npairs;
     const float* p = F32(p);
     k_sample_l1<<<(unsigned)B, kP, 0, s>>>((int)B, nullptr, src, src_off, tgt, tgt_off, seed, p + kL.w1, p + kL.b1, F32(x0),
-                                           BF(x1), F32(frame), nullptr, nullptr, nullptr);
+                                           BF(x1), nullptr, F32(frame), nullptr, nullptr, nullptr);
     if ((rc = forward_from_x1(n, B, nullptr, 1.f, false, s))) return rc;
     k_finalize<<<(unsigned)((B + 127) / 128), 128, 0, s>>>((int)B, F32(out), F32(frame), T_out);
     return cudaGetLastError() == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;

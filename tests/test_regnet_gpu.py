@@ -52,6 +52,29 @@ def test_gradient_matches_oracle(pvvc_lib, torch, B, seed):
         assert err <= GRAD_RTOL * np.linalg.norm(gr[k]) + 1e-7, (k, err, np.linalg.norm(gr[k]))
 
 
+@pytest.mark.parametrize("sizes", [(64, 192, 64), (320,)])
+def test_gradient_of_repeated_points_and_reused_buffers(pvvc_lib, torch, sizes):
+    """Clouds whose rows come twice (every pooled maximum is a tie: the first row
+    takes the gradient), over calls of several sizes on one network; same bounds."""
+    from pvvc.regnet import RegNet
+    net = RegNet(seed=3)
+    flat = net.get_params()
+    for B in sizes:
+        rng = np.random.default_rng(B)
+        half = rng.normal(0, 1, (B, 2, ro.P // 2, 3)).astype(np.float32)
+        x0 = np.concatenate([half, half], 2)
+        y = rng.normal(0, 0.5, (B, 6)).astype(np.float32)
+        g, loss = net.grad(torch.from_numpy(x0).cuda(), torch.from_numpy(y).cuda(), 4.0,
+                           stream=torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        lref, gref, _ = ro.loss_and_grad(flat, x0, y, 4.0)
+        assert abs(float(loss.item()) - lref) <= 1e-3 * abs(lref)
+        gg, gr = _blocks(g.cpu().numpy()), _blocks(gref)
+        for k in ro.DIMS:
+            err = np.linalg.norm(gg[k] - gr[k])
+            assert err <= GRAD_RTOL * np.linalg.norm(gr[k]) + 1e-7, (B, k, err, np.linalg.norm(gr[k]))
+
+
 def test_params_round_trip_and_reset(pvvc_lib, torch):
     from pvvc.regnet import RegNet
     a, b = RegNet(seed=5), RegNet(seed=6)
