@@ -142,6 +142,11 @@ struct EpiArgs {
 
 constexpr int kTileA = kBM * kBK * 2;  // 16 KB
 
+// An epilogue besides the entry point's: max(row + bias, 0) rounded to bf16 and
+// reduced over each 256 rows into C[row / 256][column] by atomicMax of keys
+// (value's bits << 16 | 255 - row % 256): the first row of the largest value.
+constexpr int kEpiReluPool = 64;
+
 // Epilogue of one 128 x BN tile: this thread's accumulator row (TMEM lane
 // `tl`'s columns) through bias / ReLU / mask into C row `row`.  A warp
 // instruction (tcgen05.ld): every lane of the warp calls it.
@@ -247,6 +252,22 @@ __device__ __forceinline__ void epilogue_warp(uint32_t tl, int row0, int M, int 
                                               ch * 8) = val;
             }
             __syncwarp();
+        }
+    } else if constexpr (EPI == kEpiReluPool) {
+#pragma unroll 1
+        for (int c0 = cbeg; c0 < cend; c0 += 32) {
+            float v[32];
+            tmem_ld32(tl + c0, v);
+            const int col = n0 + c0;
+            uint32_t mine = 0;  // the key of column `lane`
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                const __nv_bfloat16 h = __float2bfloat16_rn(fmaxf(v[j] + ep.bias[col + j], 0.f));
+                const uint32_t key = row < M ? (uint32_t)__bfloat16_as_ushort(h) << 16 | (255u - (row & 255)) : 0u;
+                const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+                if (lane == j) mine = top;
+            }
+            if (row0 < M) atomicMax(static_cast<uint32_t*>(ep.C) + (int64_t)(row0 >> 8) * ep.ldc + col + lane, mine);
         }
     } else {
         epilogue_row<BN, EPI>(tl, row, M, n0, cbeg, cend, ep);
@@ -489,6 +510,20 @@ int gemm_bf16(int32_t M, int32_t N, int32_t K, const void* A, int64_t lda, const
                   : BN == 128 ? launch_epi<128>(epi, ma, mb, M, N, K, splits, ep, s)
                               : launch_epi<64>(epi, ma, mb, M, N, K, splits, ep, s);
     return e == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;
+}
+
+// pool[m / 256][n] = max over the 256 rows of bf16(max(A B^T + bias, 0)), as keys
+// (kEpiReluPool; pool is zeroed here): the rows themselves, 268 MB at M = 524,288,
+// are neither written nor read back by a pooling kernel: 67 + 58 us before, 80 + 4
+// now.
+int gemm_relu_pool(int32_t M, int32_t K, const void* A, const void* B, const float* bias, uint32_t* pool, cudaStream_t s) {
+    constexpr int N = 256;
+    CUtensorMap ma, mb;
+    if (M % 256 || K % kBK) return PVVC_ERR_ARG;
+    if (!make_map(&ma, A, M, K, K, kBM) || !make_map(&mb, B, N, K, K, N)) return PVVC_ERR_CUDA;
+    if (cudaMemsetAsync(pool, 0, 4ull * (M / 256) * N, s) != cudaSuccess) return PVVC_ERR_CUDA;
+    EpiArgs ep{pool, N, bias, nullptr, 0, kBK, 0, 0};
+    return launch_bn<N, kEpiReluPool>(ma, mb, M, N, K, 1, ep, s) == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;
 }
 
 // C[128, 64] += A B^T over K = 64 * nkb, split over `splits`, with the operands in

@@ -9,7 +9,7 @@
 //   x0  = (p - centroid(cloud)) / s,   s = RMS radius of the source sample
 //   X1  = relu(W1 x0 + b1)      3 -> 64     CUDA cores (fused with sampling)
 //   X2  = relu(X1 W2^T + b2)   64 -> 128    tcgen05 GEMM, bf16 out
-//   Y3  = relu(X2 W3^T + b3)  128 -> 256    tcgen05 GEMM, bf16 out
+//   Y3  = relu(X2 W3^T + b3)  128 -> 256    tcgen05 GEMM, max over each cloud's rows in its epilogue
 //   G   = max over the P rows of each cloud (argmax kept); H0 = [G_src, G_tgt]
 //   H1  = relu(H0 W4^T + b4)  512 -> 256    tcgen05 GEMM
 //   H2  = relu(H1 W5^T + b5)  256 -> 128    tcgen05 GEMM
@@ -39,6 +39,7 @@ namespace pvvc {
 int gemm_bf16(int32_t M, int32_t N, int32_t K, const void* A, int64_t lda, const void* B, int64_t ldb, void* C,
               int64_t ldc, const float* bias, const void* aux, int64_t ldaux, int32_t epi, int32_t splits,
               cudaStream_t s);
+int gemm_relu_pool(int32_t M, int32_t K, const void* A, const void* B, const float* bias, uint32_t* pool, cudaStream_t s);
 int gemm_bf16_blocked(int32_t nkb, const void* A, const void* B, float* C, int64_t ldc, int32_t splits, cudaStream_t s);
 
 namespace {
@@ -219,22 +220,15 @@ __global__ void __launch_bounds__(256) k_l1(int64_t rows, const float* __restric
         }
 }
 
-// max over each cloud's P rows of Y3 (first maximum), into H0 = [G_src | G_tgt]
-__global__ void __launch_bounds__(256) k_pool(const __nv_bfloat16* __restrict__ y3, __nv_bfloat16* __restrict__ h0,
-                                              int32_t* __restrict__ amax) {
+// The max over each cloud's P rows (first maximum) from layer 3's keys, into
+// H0 = [G_src | G_tgt] and the rows' indices
+__global__ void __launch_bounds__(256) k_pool_out(const uint32_t* __restrict__ pool, __nv_bfloat16* __restrict__ h0,
+                                                  int32_t* __restrict__ amax) {
+    static_assert(kP == 256, "a key holds the row in 8 bits");
     const int c = blockIdx.x, ch = threadIdx.x;
-    const __nv_bfloat16* base = y3 + (int64_t)c * kP * kD3 + ch;
-    float best = __bfloat162float(base[0]);
-    int arg = 0;
-    for (int r = 1; r < kP; ++r) {
-        const float v = __bfloat162float(base[(int64_t)r * kD3]);
-        if (v > best) {
-            best = v;
-            arg = r;
-        }
-    }
-    h0[(int64_t)(c >> 1) * kH0 + (c & 1) * kD3 + ch] = __float2bfloat16_rn(best);
-    amax[c * kD3 + ch] = arg;
+    const uint32_t key = pool[c * kD3 + ch];
+    h0[(int64_t)(c >> 1) * kH0 + (c & 1) * kD3 + ch] = __ushort_as_bfloat16((unsigned short)(key >> 16));
+    amax[c * kD3 + ch] = 255 - (int32_t)(key & 255u);
 }
 
 // Output layer, loss and its gradient.  One pair per block of 128 threads.
@@ -658,7 +652,7 @@ struct pvvc_regnet {
     int64_t step = 0;
     // activations and scratch for up to `cap` pairs
     int64_t cap = 0;
-    DevBuf x0, x1, x2, y3, h0, amax, h1, h2, out, frame, y, dh2, dh1, dh0, dy2, dy1, loss, ids;
+    DevBuf x0, x1, x2, pool, h0, amax, h1, h2, out, frame, y, dh2, dh1, dh0, dy2, dy1, loss, ids;
     DevBuf x1t, dy2t;  // transposes (the weight gradient of layer 2)
     DevBuf ta, tb;     // ... of the head layers' operands
     SideStream side;   // the weight gradients that nothing else of the pass waits for
@@ -677,7 +671,7 @@ int ensure_cap(pvvc_regnet* n, int64_t B) {
     if (B <= n->cap) return PVVC_OK;
     const int64_t M = 2 * B * kP;
     bool ok = n->x0.ensure(12 * M) == cudaSuccess && n->x1.ensure(2 * M * kD1) == cudaSuccess &&
-              n->x2.ensure(2 * M * kD2) == cudaSuccess && n->y3.ensure(2 * M * kD3) == cudaSuccess &&
+              n->x2.ensure(2 * M * kD2) == cudaSuccess && n->pool.ensure(4 * 2 * B * kD3) == cudaSuccess &&
               n->h0.ensure(2 * B * kH0) == cudaSuccess && n->amax.ensure(4 * 2 * B * kD3) == cudaSuccess &&
               n->h1.ensure(2 * B * kH1) == cudaSuccess && n->h2.ensure(2 * B * kH2) == cudaSuccess &&
               n->out.ensure(4 * B * kOut) == cudaSuccess && n->frame.ensure(4 * B * 7) == cudaSuccess &&
@@ -722,10 +716,9 @@ int forward_from_x1(pvvc_regnet* n, int64_t B, const float* y, float lambda_w, b
     if ((rc = gemm_bf16((int32_t)M, kD2, kD1, BF(x1), kD1, BF(w2b), kD1, BF(x2), kD2, p + kL.b2, nullptr, 0,
                         PVVC_GEMM_BIAS_RELU_BF16, 1, s)))
         return rc;
-    if ((rc = gemm_bf16((int32_t)M, kD3, kD2, BF(x2), kD2, BF(w3b), kD2, BF(y3), kD3, p + kL.b3, nullptr, 0,
-                        PVVC_GEMM_BIAS_RELU_BF16, 1, s)))
-        return rc;
-    k_pool<<<(unsigned)(2 * B), kD3, 0, s>>>(BF(y3), BF(h0), static_cast<int32_t*>(n->amax.p));
+    uint32_t* pool = static_cast<uint32_t*>(n->pool.p);
+    if ((rc = gemm_relu_pool((int32_t)M, kD2, BF(x2), BF(w3b), p + kL.b3, pool, s))) return rc;
+    k_pool_out<<<(unsigned)(2 * B), kD3, 0, s>>>(pool, BF(h0), static_cast<int32_t*>(n->amax.p));
     if ((rc = gemm_bf16((int32_t)B, kH1, kH0, BF(h0), kH0, BF(w4b), kH0, BF(h1), kH1, p + kL.b4, nullptr, 0,
                         PVVC_GEMM_BIAS_RELU_BF16, 1, s)))
         return rc;
