@@ -88,12 +88,15 @@ ZFN uint64_t le64(const uint8_t* p) { return (uint64_t)le32(p) | ((uint64_t)le32
 // going negative is libzstd's overflow state.  The next bits sit
 // left-aligned in a 64-bit container: a read is one shift out of its top,
 // and 32 more bits are taken from the stream whenever fewer than a read
-// needs remain.
+// needs remain.  Those were loaded a refill earlier (`ahead`): a load is then
+// never waited for by the symbol that needs it (the longest payload of a GoP, 5
+// KB: 266 us with the load in the refill, 230 ahead of it).
 struct BackBits {
     const uint8_t* p;
     int32_t n;
     int32_t pos;    // stream bits [0, pos) not yet consumed
     int32_t valid;  // container bits (from the top) that hold stream bits pos-1, pos-2, ...
+    uint32_t ahead;  // stream bits [pos - valid - 32, pos - valid)
     uint64_t c;
 
     // stream bits [b0, b0 + 32), bit b0 + 31 as the MSB; bits outside the stream are zero
@@ -101,7 +104,14 @@ struct BackBits {
         const int32_t k0 = b0 >> 3;  // floor
         uint64_t v = 0;
         if (k0 >= 0 && k0 + 5 <= n) {
+#if defined(__CUDA_ARCH__)
+            // the two aligned words that hold the five bytes (each holds one of them at least)
+            const uintptr_t a = reinterpret_cast<uintptr_t>(p + k0);
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+            v = ((uint64_t)w[0] | ((uint64_t)w[1] << 32)) >> (8 * (a & 3));
+#else
             v = (uint64_t)le32(p + k0) | ((uint64_t)p[k0 + 4] << 32);
+#endif
         } else {
             for (int i = 4; i >= 0; --i) {
                 const int32_t k = k0 + i;
@@ -116,19 +126,40 @@ struct BackBits {
             valid = 64;
             return;
         }
-        c |= (uint64_t)bits32(lo - 32) << (32 - valid);
+        c |= (uint64_t)ahead << (32 - valid);
         valid += 32;
+        ahead = bits32(lo - 64);
+    }
+    // stream bits [pos - 64, pos), the first one read as the MSB of hi; pos >= 64
+    ZFN void window(uint32_t& hi, uint32_t& lo) const {
+        const int32_t b0 = pos - 64, k0 = b0 >> 3;
+#if defined(__CUDA_ARCH__)
+        // three aligned words, each with a byte of the window (the end mark lies above it)
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p + k0);
+        const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+        const uint32_t sh = 8 * (uint32_t)(a & 3) + (uint32_t)(b0 & 7), m = w[1];
+        lo = __funnelshift_r(w[0], m, sh);
+        hi = __funnelshift_r(m, w[2], sh);
+#else
+        lo = bits32(b0);
+        hi = bits32(b0 + 32);
+        (void)k0;
+#endif
+    }
+    ZFN void seek(int32_t at) {
+        pos = at;
+        c = 0;
+        valid = 0;
+        ahead = bits32(pos - 32);
+        fill();
+        fill();
     }
     // false: empty stream or a zero last byte (BIT_initDStream's errors)
     ZFN bool init(const uint8_t* s, int64_t len) {
         p = s;
         n = (int32_t)len;
         if (len <= 0 || s[len - 1] == 0) return false;
-        pos = 8 * (int32_t)(len - 1) + highbit(s[len - 1]);
-        c = 0;
-        valid = 0;
-        fill();
-        fill();
+        seek(8 * (int32_t)(len - 1) + highbit(s[len - 1]));
         return true;
     }
     ZFN uint32_t peek(int nb) {  // nb <= 32
@@ -403,10 +434,39 @@ ZFN void fill_huf(Shared& sh, int nsym, int log, int lane, int nl) {
 // HUF_decompress1X1_usingDTable): each step looks up the next `log` bits and
 // consumes the entry's code length.  The stream must end exactly at its first
 // bit.  false: bad stream.
+//
+// While 64 bits are left, four symbols (48 bits at most) come from one window of
+// them without a check between: the four streams' lanes stay in step, and a symbol
+// is a shift, a table read and a funnel shift (the 5 KB payload: 230 us by single reads, with
+// some lane refilling at most of them; 172).
 ZFN bool huf_stream(const Shared& sh, int log, const uint8_t* s, int64_t len, uint8_t* out, uint32_t count) {
     BackBits br;
     if (!br.init(s, len)) return false;
-    for (uint32_t i = 0; i < count; ++i) {
+    uint32_t i = 0;
+    if (br.pos >= 64) {
+        for (; br.pos >= 64 && i + 4 <= count; i += 4) {
+            uint32_t hi, lo;
+            br.window(hi, lo);
+            int32_t used = 0;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t e = sh.huf[hi >> (32 - log)], nb = e & 15;
+#if defined(__CUDA_ARCH__)
+                hi = __funnelshift_l(lo, hi, nb);
+#else
+                hi = (hi << nb) | (nb ? lo >> (32 - nb) : 0u);
+#endif
+                lo <<= nb;
+                used += (int32_t)nb;
+                out[i + k] = (uint8_t)(e >> 4);
+            }
+            br.pos -= used;
+        }
+        br.seek(br.pos);
+    }
+    for (; i < count; ++i) {
         const uint16_t e = sh.huf[br.peek(log)];
         br.skip(e & 15);
         out[i] = (uint8_t)(e >> 4);
@@ -456,12 +516,18 @@ struct FrameState {
 // dst + o (each chunk is read before it is written).
 ZFN void put_lits(uint8_t* dst, uint64_t o, const uint8_t* from, uint8_t rle, int kind, uint32_t n, int lane, int nl) {
     if (kind == 2) {
-        for (uint32_t b = 0; b < n; b += (uint32_t)nl) {
-            const uint32_t i = b + (uint32_t)lane;
-            uint8_t v = 0;
-            if (i < n) v = from[i];
+        constexpr int kAhead = 8;  // bytes a lane reads before any is written (the 5 KB payload: 172 us with one, 125)
+        for (uint32_t b = 0; b < n; b += kAhead * (uint32_t)nl) {
+            uint8_t v[kAhead];
+            for (int k = 0; k < kAhead; ++k) {
+                const uint32_t i = b + (uint32_t)(k * nl + lane);
+                v[k] = i < n ? from[i] : 0;
+            }
             wsync();
-            if (i < n) dst[o + i] = v;
+            for (int k = 0; k < kAhead; ++k) {
+                const uint32_t i = b + (uint32_t)(k * nl + lane);
+                if (i < n) dst[o + i] = v[k];
+            }
         }
     } else {
         for (uint32_t i = (uint32_t)lane; i < n; i += (uint32_t)nl) dst[o + i] = kind ? rle : from[i];

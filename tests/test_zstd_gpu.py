@@ -77,3 +77,21 @@ def test_gpu_inflate_no_jobs_and_bad_args(pvvc_lib, torch):
     assert L.pvvc_zstd_inflate_batch(0, None, None, None, None, None, None, None, None, None) == 0
     assert L.pvvc_zstd_inflate_batch(-1, None, None, None, None, None, None, None, None, None) != 0
     assert L.pvvc_zstd_inflate_batch(1, None, None, None, None, None, None, None, None, None) != 0
+
+
+@pytest.mark.parametrize("njobs", [33, 4000])
+def test_gpu_inflate_size_classes_and_stream_tails(pvvc_lib, torch, njobs):
+    """Few jobs and more than fit on the device at once (then by size class, the
+    longest first), of skewed bytes (four Huffman streams) whose literal counts
+    cover every remainder of four symbols a step, around the classes' limits."""
+    rng = np.random.default_rng(njobs)
+    p = np.exp(-np.arange(256) / 40.0)
+    pool = rng.choice(256, 1 << 17, p=p / p.sum()).astype(np.uint8).tobytes()
+    sizes = [0, 1, 5, 6, 7, 62, 63, 64, 65, 1023, 1024, 1025, 2047, 2048, 4095, 4096, 4097, 9000]
+    sizes += [int(v) for v in rng.integers(6, 7000, njobs - len(sizes))]
+    rng.shuffle(sizes)
+    datas = [pool[o:o + n] for o, n in zip(rng.integers(0, (1 << 17) - 9000, njobs), sizes)]
+    uniq = [zr.compress(d, 3 if i % 2 else 19) for i, d in enumerate(datas)]
+    outs, st = pvvc_lib.zstd.inflate_device(uniq, [len(d) for d in datas])
+    assert st == [0] * njobs
+    assert all(o == d for o, d in zip(outs, datas))
