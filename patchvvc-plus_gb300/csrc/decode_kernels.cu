@@ -10,9 +10,9 @@
 //           fused dequantisation, written un-reversed as Y|U|V planes.
 //           Restates RLGRDecoder::Decode (src/common/entropy_codec.cc:163-283)
 //           and the dequantisation of invert_raht_octree.cc:63-69.
-//   k_raht  one CTA per slice: level-synchronous inverse RAHT (7 butterflies
-//           per internal node, octree_base.cc:84-100,186-206) with the level
-//           signal in shared memory, fused with the reference-colour add
+//   k_raht_slice, k_raht_few, k_raht_group  a slice or a group of slices that
+//           share a tree: level-synchronous inverse RAHT (7 butterflies
+//           per internal node, octree_base.cc:84-100,186-206), fused with the reference-colour add
 //           (invert_raht_octree.cc:304-311), YUV->RGB (common.h:154-158) and
 //           the rigid transform (pvvc_decompression.cc:141-150).
 //
