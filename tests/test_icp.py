@@ -163,6 +163,41 @@ def test_gpu_icp_same_for_any_cta_size(pvvc_lib):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("noalloc", [False, True])
+def test_gpu_icp_size_classes(pvvc_lib, noalloc):
+    """More pairs than SMs, sources of 0 to 6,000 points around the limits of the
+    size classes, in a shuffled order: every pair is run once, and its results
+    are those of a batch that fits on the device, bit for bit."""
+    import ctypes as C
+    import torch
+    from pvvc import _lib as L
+    from pvvc.icp import IcpBatch, Pairs
+    rng = np.random.default_rng(4)
+    sizes = [0, 1, 3, 724, 725, 1024, 1025, 1448, 1449, 2047, 2048, 2896, 2897, 4095, 4096, 5792, 5793, 6000]
+    sizes += [int(v) for v in rng.integers(3, 700, 40)]
+    n, few = torch.cuda.get_device_properties(0).multi_processor_count + 40, 58
+    order = rng.permutation(np.arange(n) % few)
+    src = [rng.uniform(0, 40, (v, 3)).astype(np.float32) for v in sizes]
+    tgt = [(s + rng.normal(0, 0.4, s.shape)).astype(np.float32)[: max(len(s), 1)] if len(s) else np.ones((3, 3), np.float32)
+           for s in src]
+
+    def results(ids):
+        b = IcpBatch(Pairs([src[i] for i in ids], [tgt[i] for i in ids], np.tile(np.eye(4), (len(ids), 1, 1))))
+        prm = L.IcpParams(1e6, 10, 0.0, 0.0, 1e-6)
+        if noalloc:
+            L.check(L.lib().pvvc_icp_batch_noalloc(b.n, b.src.data_ptr(), b.soff.data_ptr(), b.tgt.data_ptr(), b.toff.data_ptr(),
+                                                   None, C.byref(prm), b.T.data_ptr(), b.mse.data_ptr(), b.iters.data_ptr(),
+                                                   b.conv.data_ptr(), b.nt, torch.cuda.current_stream().cuda_stream), "noalloc")
+        else:
+            b.run(max_iter=10)
+        return [np.asarray(v).reshape(len(ids), -1) for v in b.results()]
+
+    want = results(range(few))
+    for g, w in zip(results(order), want):
+        assert np.array_equal(g, w[order], equal_nan=g.dtype.kind == "f")
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("flat", [1.0, 1e-3, 0.0])
 def test_gpu_icp_flat_patches(pvvc_lib, oracle, flat):
     """A patch and its moved copy, flattened to a plane: the covariance's
