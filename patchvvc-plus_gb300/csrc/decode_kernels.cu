@@ -864,6 +864,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rlgr_win(const SliceWork* __rest
         }
         if (mn == total) break;
     }
+    br.drain();  // a lane that finished last has copies of its last two stage() calls in flight
 }
 
 // ---------------------------------------------------------------------------

@@ -539,3 +539,32 @@ def test_failed_intra_fails_its_group_only(pvvc_lib, torch, streams, nframes):
         for s in np.flatnonzero(~hit):
             a, b = int(bad.out_off[s]), int(bad.out_off[s]) + int(bad.size[s])
             assert np.array_equal(xyz[a:b], want[0][a:b]) and np.array_equal(rgb[a:b], want[1][a:b]), s
+
+
+def _window_batch(pvvc, torch, parsed):
+    """The GoP often enough that its groups are as many as the device has SMs
+    (from there on they are decoded by the windowed RLGR): batch, slots."""
+    streams = -(-torch.cuda.get_device_properties(0).multi_processor_count // 8)
+    return pvvc.concat_batches([pvvc.pack_frames(parsed)] * streams, slot_stride=8), 8 * streams
+
+
+@pytest.mark.parametrize("block", [32, 64, 128, 256])
+def test_windowed_payloads_longer_than_their_symbols(pvvc_lib, torch, block):
+    """Colour payloads with kilobytes after their last symbol, so that every lane of
+    the windowed RLGR ends with blocks of its payload still being copied: decode
+    after decode, the outputs are those of the payloads without them."""
+    parsed = [pvvc_lib.parse_frame(b) for b in _large_value_frames(pvvc_lib, 17)]
+    batch, nslots = _window_batch(pvvc_lib, torch, parsed)
+    tune = (3, 4, block, -1, -1, 32)  # every group windowed
+    info = pvvc_lib.Plan(batch, tune=tune).info()
+    assert info["clear_bytes"] == 0 and info["group_ctas"] > 0 and info["singles_a"] == 0  # no per-slice RLGR
+    dec = pvvc_lib.Decoder(nslots=nslots, max_leaves=4096)
+    want = decode_batch(torch, pvvc_lib, dec, batch, tune=tune)
+    assert (want[2] == 0).all()
+    rng = np.random.default_rng(2)
+    for f in parsed:
+        f.color = [c + rng.integers(0, 256, int(rng.integers(500, 5000)), dtype=np.uint8).tobytes() for c in f.color]
+    longer, _ = _window_batch(pvvc_lib, torch, parsed)
+    for _ in range(3):
+        for a, b in zip(decode_batch(torch, pvvc_lib, dec, longer, tune=tune), want):
+            assert np.array_equal(a, b)
