@@ -347,10 +347,12 @@ struct BitReader {
         }
         s1 = s2 = s3 = landed = sp;
     }
-    // a lane without a slice (it takes part in stage() only)
-    __device__ __forceinline__ void idle() {
+    // a lane without a slice: it takes part in stage(), and reads words of its
+    // own ring that it never uses
+    __device__ __forceinline__ void idle(const uint4* ring0) {
         first = nullptr;
-        nblk = ring = hi = lo = nx = o = wi = sp = s1 = s2 = s3 = landed = 0;
+        ring = (uint32_t)__cvta_generic_to_shared(ring0);
+        nblk = hi = lo = nx = o = wi = sp = s1 = s2 = s3 = landed = 0;
     }
     __device__ __forceinline__ void init(const uint8_t* payload, uint64_t off, uint32_t nbytes, uint4* ring0) {
         first = reinterpret_cast<const uint4*>(payload + (off & ~15ull));
@@ -579,7 +581,7 @@ __global__ void __launch_bounds__(T) k_rlgr(const SliceWork* __restrict__ work, 
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int t = (g >> 5) * LANES + lane;
     BitReader br;
-    br.idle();
+    br.idle(s_ring + threadIdx.x * kRing);
     uint32_t N = 0, rem = 0;   // symbols of a plane; left in the current plane
     uint32_t qp = 0;
     int plane = 0;
@@ -721,7 +723,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_rlgr_win(const SliceWork* __rest
     for (int i = lane; i < WROWS * 8; i += 32) reinterpret_cast<float4*>(win)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     __syncwarp();  // rows are cleared by all lanes, then written by their owners
     BitReader br;
-    br.idle();
+    br.idle(s_dyn + threadIdx.x * kRing);
     bool live = false, pend = false;
     uint32_t qp = 0;
     uint32_t s = total;             // stream position of this lane's next symbol (total: done)

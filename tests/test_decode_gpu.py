@@ -568,3 +568,20 @@ def test_windowed_payloads_longer_than_their_symbols(pvvc_lib, torch, block):
     for _ in range(3):
         for a, b in zip(decode_batch(torch, pvvc_lib, dec, longer, tune=tune), want):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("lanes", [8, 16, 32])
+@pytest.mark.parametrize("nframes", [1, 2, 17])
+def test_partly_idle_warps(pvvc_lib, torch, lanes, nframes):
+    """Batches that leave most lanes of an RLGR warp without a slice (8 x nframes
+    slices, a quarter of them in the long launch), for every packing of the long
+    launch's warps: the outputs of the default packing."""
+    parsed = [pvvc_lib.parse_frame(b) for b in _large_value_frames(pvvc_lib, nframes)]
+    batch = pvvc_lib.pack_frames(parsed)
+    dec = pvvc_lib.Decoder(nslots=8, max_leaves=4096)
+    want = decode_batch(torch, pvvc_lib, dec, batch)
+    assert (want[2] == 0).all()
+    for block in (32, 256):
+        got = decode_batch(torch, pvvc_lib, dec, batch, tune=(3, 4, block, 16, 50, lanes))
+        for a, b in zip(got, want):
+            assert np.array_equal(a, b)
