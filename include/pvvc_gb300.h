@@ -506,13 +506,15 @@ int pvvc_regnet_set_params(pvvc_regnet* net, const float* host, int64_t count);
 /* One training step on the pairs pair_ids[0..npairs) of a device dataset
  * (clouds as for pvvc_icp_batch; T_label [*,16] row-major converged ICP
  * transforms, omega_label [*,3] their axis-angle): sample, forward, loss,
- * backward, AdamW.  loss_out: device float (or NULL).  Stream-ordered. */
+ * backward, AdamW.  npairs: a multiple of 64 (PVVC_ERR_ARG otherwise, nothing
+ * queued).  loss_out: device float (or NULL).  Stream-ordered. */
 int pvvc_regnet_train_step(pvvc_regnet* net, int32_t npairs, const int32_t* pair_ids, const float* src,
                            const uint32_t* src_off, const float* tgt, const uint32_t* tgt_off, const float* T_label,
                            const float* omega_label, uint64_t seed, const pvvc_adamw* opt, float* loss_out, void* stream);
 /* Gradient of the loss for given normalised inputs x0 [npairs*2*256*3] (pair
  * b's source rows then target rows) and targets y [npairs*6]: grad_out
- * [param_count] (device), loss_out (device float).  No update. */
+ * [param_count] (device), loss_out (device float).  npairs as for a training
+ * step.  No update. */
 int pvvc_regnet_grad(pvvc_regnet* net, int32_t npairs, const float* x0, const float* y, float lambda_w, float* grad_out,
                      float* loss_out, void* stream);
 /* Proposed transforms T_out [npairs*16] (row-major) for every pair. */

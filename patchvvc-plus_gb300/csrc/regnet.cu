@@ -750,6 +750,10 @@ int weight_grad(int64_t rows, int dout, int din, const __nv_bfloat16* dy, const 
                      splits, s);
 }
 
+// The weight gradients are GEMMs over the pairs in blocks of 64 (gemm_bf16's K): a
+// call with another count is refused before anything is queued.
+constexpr int kTrainBlock = 64;
+
 // Backward after forward_from_x1 (k_head wrote dH2, dW6, db6).  x0 rows for dW1.
 int backward(pvvc_regnet* n, int64_t B, cudaStream_t s) {
     const int64_t M = 2 * B * kP;
@@ -758,7 +762,13 @@ int backward(pvvc_regnet* n, int64_t B, cudaStream_t s) {
     // The chain dH1, dH0, dY2, dY1 on this stream; the weight gradients of the head
     // layers (small kernels, 100 us of launches one after another) and of layer 3
     // (gathers, bound by latency) beside it on the side stream.
+    // Whatever ends the pass early, the calling stream waits for the side stream:
+    // its kernels add into the gradient, which the next call clears.
     const SideStream& w = n->side;
+    auto joined = [&](int rc) {
+        const bool ok = cudaEventRecord(w.join, w.s) == cudaSuccess && cudaStreamWaitEvent(s, w.join, 0) == cudaSuccess;
+        return rc ? rc : ok ? PVVC_OK : PVVC_ERR_CUDA;
+    };
     if ((rc = gemm_bf16((int32_t)B, kH1, kH2, BF(dh2), kH2, BF(w5t), kH2, BF(dh1), kH1, nullptr, BF(h1), kH1,
                         PVVC_GEMM_MASK_BF16, 1, s)))
         return rc;
@@ -769,24 +779,23 @@ int backward(pvvc_regnet* n, int64_t B, cudaStream_t s) {
     // dW3, db3; dW4, db4; dW5, db5
     k_pool_bwd_w3<<<dim3(kD3, kPoolParts), kD2, 0, w.s>>>((int)(2 * B), F32(dh0), BF(h0), static_cast<int32_t*>(n->amax.p),
                                                           BF(x2), g + kL.w3, g + kL.b3);
-    if ((rc = weight_grad(B, kH1, kH0, BF(dh1), BF(h0), BF(ta), BF(tb), g + kL.w4, w.s))) return rc;
+    if ((rc = weight_grad(B, kH1, kH0, BF(dh1), BF(h0), BF(ta), BF(tb), g + kL.w4, w.s))) return joined(rc);
     k_colsum<<<(unsigned)((B + 63) / 64), 256, 0, w.s>>>(BF(dh1), B, kH1, 64, g + kL.b4);
-    if ((rc = weight_grad(B, kH2, kH1, BF(dh2), BF(h1), BF(ta), BF(tb), g + kL.w5, w.s))) return rc;
+    if ((rc = weight_grad(B, kH2, kH1, BF(dh2), BF(h1), BF(ta), BF(tb), g + kL.w5, w.s))) return joined(rc);
     k_colsum<<<(unsigned)((B + 63) / 64), 128, 0, w.s>>>(BF(dh2), B, kH2, 64, g + kL.b5);
     // max-pool + layer 3 (sparse): dY2
     k_pool_bwd_x2<<<(unsigned)(2 * B), 256, 0, s>>>(F32(dh0), BF(h0), static_cast<int32_t*>(n->amax.p), BF(w3b),
                                                                BF(x2), BF(dy2), BF(dy2t), F32(part));
     // layer 2: dW2 (x1t: written with X1), db2, dY1
     k_colsum_parts<<<dim3(kD2 / 32, (unsigned)((2 * B + 63) / 64)), dim3(32, 8), 0, s>>>(F32(part), 2 * B, kD2, 64, g + kL.b2);
-    if ((rc = gemm_bf16_blocked((int32_t)(M / 64), BF(dy2t), BF(x1t), g + kL.w2, kD1, sm_count(), s))) return rc;
+    if ((rc = gemm_bf16_blocked((int32_t)(M / 64), BF(dy2t), BF(x1t), g + kL.w2, kD1, sm_count(), s))) return joined(rc);
     if ((rc = gemm_bf16((int32_t)M, kD1, kD2, BF(dy2), kD2, BF(w2t), kD2, BF(dy1), kD1, nullptr, BF(x1), kD1,
                         PVVC_GEMM_MASK_BF16, 1, s)))
-        return rc;
+        return joined(rc);
     // layer 1
     const int64_t per = std::max<int64_t>(512, (M + 4 * sm_count() - 1) / (4 * sm_count()));
     k_bwd_w1<<<(unsigned)((M + per - 1) / per), 256, 0, s>>>(BF(dy1), F32(x0), M, per, g + kL.w1, g + kL.b1);
-    if (cudaEventRecord(w.join, w.s) != cudaSuccess || cudaStreamWaitEvent(s, w.join, 0) != cudaSuccess) return PVVC_ERR_CUDA;
-    return cudaGetLastError() == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA;
+    return joined(cudaGetLastError() == cudaSuccess ? PVVC_OK : PVVC_ERR_CUDA);
 }
 
 }  // namespace
@@ -855,7 +864,7 @@ extern "C" int pvvc_regnet_set_params(pvvc_regnet* n, const float* host, int64_t
 
 extern "C" int pvvc_regnet_grad(pvvc_regnet* n, int32_t npairs, const float* x0, const float* y, float lambda_w,
                                 float* grad_out, float* loss_out, void* stream) {
-    if (!n || npairs <= 0 || !x0 || !y) return PVVC_ERR_ARG;
+    if (!n || npairs <= 0 || npairs % kTrainBlock || !x0 || !y) return PVVC_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     int rc = ensure_cap(n, npairs);
     if (rc) return rc;
@@ -879,7 +888,7 @@ extern "C" int pvvc_regnet_train_step(pvvc_regnet* n, int32_t npairs, const int3
                                       const uint32_t* src_off, const float* tgt, const uint32_t* tgt_off, const float* T_label,
                                       const float* omega_label, uint64_t seed, const pvvc_adamw* opt, float* loss_out,
                                       void* stream) {
-    if (!n || npairs <= 0 || !pair_ids || !src || !src_off || !tgt || !tgt_off || !T_label || !omega_label || !opt)
+    if (!n || npairs <= 0 || npairs % kTrainBlock || !pair_ids || !src || !src_off || !tgt || !tgt_off || !T_label || !omega_label || !opt)
         return PVVC_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     int rc = ensure_cap(n, npairs);

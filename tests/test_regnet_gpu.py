@@ -75,6 +75,53 @@ def test_gradient_of_repeated_points_and_reused_buffers(pvvc_lib, torch, sizes):
             assert err <= GRAD_RTOL * np.linalg.norm(gr[k]) + 1e-7, (B, k, err, np.linalg.norm(gr[k]))
 
 
+def test_refused_size_leaves_the_next_gradient_alone(pvvc_lib, torch):
+    """A batch that is no multiple of 64 is refused with nothing of it left on
+    the device: gradients of a good batch queued right behind it, on the same
+    stream and without a synchronisation, and a captured one, keep the bounds
+    above."""
+    from pvvc.regnet import AdamW, RegNet
+    net = RegNet(seed=4)
+    flat = net.get_params()
+    rng = np.random.default_rng(9)
+    x0 = rng.normal(0, 1, (128, 2, ro.P, 3)).astype(np.float32)
+    y = rng.normal(0, 0.5, (128, 6)).astype(np.float32)
+    dx, dy = torch.from_numpy(x0).cuda(), torch.from_numpy(y).cuda()
+    _, gref, _ = ro.loss_and_grad(flat, x0, y, 4.0)
+    gr = _blocks(gref)
+    sp = torch.cuda.current_stream().cuda_stream
+    runs = []
+    for it in range(20):
+        for bad in (100, 1, 65):
+            with pytest.raises(pvvc_lib.PvvcError) as e:
+                net.grad(dx[:bad], dy[:bad], 4.0, stream=sp)
+            assert e.value.status == 1
+        runs.append(net.grad(dx, dy, 4.0, stream=sp)[0])
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        with pytest.raises(pvvc_lib.PvvcError):
+            net.grad(dx[:100], dy[:100], 4.0, stream=s.cuda_stream)
+        runs.append(net.grad(dx, dy, 4.0, stream=s.cuda_stream)[0])
+    graph.replay()
+    torch.cuda.synchronize()
+    for it, g in enumerate(runs):
+        gg = _blocks(g.cpu().numpy())
+        for k in ro.DIMS:
+            err = np.linalg.norm(gg[k] - gr[k])
+            assert err <= GRAD_RTOL * np.linalg.norm(gr[k]) + 1e-7, (it, k, err, np.linalg.norm(gr[k]))
+    # the training step refuses the same sizes and leaves the parameters as they are
+    _, _, data, _ = _labelled(pvvc_lib, torch, 128, seed=5, synth_seed=6)
+    opt = AdamW(1e-3, 0.9, 0.999, 1e-8, 1e-4, 4.0)
+    for bad in (100, 1, 65):
+        with pytest.raises(pvvc_lib.PvvcError) as e:
+            net.train_step(data, torch.arange(bad, dtype=torch.int32, device="cuda"), seed=0, opt=opt, stream=sp)
+        assert e.value.status == 1
+    torch.cuda.synchronize()
+    assert np.array_equal(net.get_params(), flat)
+
+
 def test_params_round_trip_and_reset(pvvc_lib, torch):
     from pvvc.regnet import RegNet
     a, b = RegNet(seed=5), RegNet(seed=6)
