@@ -215,9 +215,11 @@ __global__ void __launch_bounds__(T) k_tree(const SliceWork* __restrict__ work, 
             running += tot;
         }
     }
-    // a well-formed tree codes exactly one coefficient per leaf; an empty
-    // occupancy byte breaks that and would send reads past the planes
-    if (running != count) {
+    // A well-formed tree codes exactly one coefficient per leaf, and none of its
+    // levels is wider than its leaves.  Empty occupancy bytes can break either:
+    // reads would go past the planes, and writes past the level buffers, which
+    // are sized by the leaves.
+    if (running != count || max_w > count) {
         if (tid == 0) tstatus[item] = PVVC_ERR_GEOMETRY;
         return;
     }

@@ -585,3 +585,57 @@ def test_partly_idle_warps(pvvc_lib, torch, lanes, nframes):
         got = decode_batch(torch, pvvc_lib, dec, batch, tune=(3, 4, block, 16, 50, lanes))
         for a, b in zip(got, want):
             assert np.array_equal(a, b)
+
+
+def _crafted_tree(levels, rng_half=64.0):
+    """Geometry payload of a tree given as the occupancy bytes of each level, and
+    its leaf count."""
+    n = 1
+    for b in levels:
+        assert len(b) == n
+        n = sum(bin(x).count("1") for x in b)
+    head = np.array([32.0] * 3 + [rng_half] * 3, ">f4").tobytes()
+    return head + bytes([len(levels) + 1]) + b"".join(bytes(b) for b in levels), n
+
+
+def _crafted_frames(pvvc, oracle, trees, nframes):
+    """Frames of one patch per tree (frame 0 intra), random colour symbols."""
+    rng = np.random.default_rng(8)
+    geos, ns = zip(*[_crafted_tree(t) for t in trees])
+    m = len(trees)
+    eye = np.tile(np.eye(4, dtype=np.float32).reshape(16), (m, 1))
+    return [pvvc.Frame(f, np.arange(m, dtype=np.int32), np.full(m, 1 if f == 0 else 3, np.uint8), np.array(ns, np.uint32),
+                       np.full(m, 8, np.uint8), eye, [g if f == 0 else b"" for g in geos],
+                       [oracle.rlgr_encode(rng.integers(-40, 41, 3 * n)) for n in ns]) for f in range(nframes)]
+
+
+_FULL = [[0xFF], [0xFF] * 8, [0xFF] * 64]
+_WIDE = [[0xFF], [0x80] + [0] * 7]                      # 1 leaf under a level of 8 nodes
+_WIDE2 = [[0xFF], [0xFF] * 8, [0x81] + [0] * 63, [0xFF] * 2]  # 16 leaves, 64 nodes
+
+
+@pytest.mark.parametrize("nframes", [1, 2, 20])
+@pytest.mark.parametrize("streams", [1, 60])
+def test_tree_wider_than_its_leaves_is_malformed(pvvc_lib, oracle, torch, nframes, streams):
+    """Empty occupancy bytes that leave a level wider than the leaves: the level
+    buffers are sized by the leaves, so the slice is refused as malformed geometry
+    and its other frames have no reference; the patches beside it decode."""
+    frames = _crafted_frames(pvvc_lib, oracle, [_FULL, _WIDE, _FULL, _WIDE2], nframes)
+    batch = pvvc_lib.concat_batches([pvvc_lib.pack_frames(frames)] * streams, slot_stride=4)
+    dec = pvvc_lib.Decoder(nslots=4 * streams, max_leaves=4096)
+    xyz, rgb, st = decode_batch(torch, pvvc_lib, dec, batch)
+    wide = batch.slot % 2 == 1
+    assert (st[wide & (batch.type == 1)] == 3).all() and (st[wide & (batch.type == 3)] == 5).all() and (st[~wide] == 0).all()
+    good = _crafted_frames(pvvc_lib, oracle, [_FULL, _WIDE, _FULL, _WIDE2], nframes)
+    dec4 = [oracle.decoder() for _ in range(4)]
+    for f, fr in enumerate(good):
+        a = int(batch.frame_first_point[f])
+        ox, orgb, ost = oracle.decode_frame(dec4, fr, nthreads=1)
+        at = 0
+        for i in range(fr.n):
+            n = int(fr.size[i])
+            if i % 2 == 0:
+                yuv = dec4[i].get_patch()[1]
+                assert np.array_equal(xyz[a + at:a + at + n].view(np.uint32), ox[at:at + n].view(np.uint32))
+                assert rgb_matches(rgb[a + at:a + at + n], orgb[at:at + n], yuv).all()
+            at += n
