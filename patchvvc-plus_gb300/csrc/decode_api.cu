@@ -582,6 +582,21 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         p->idx.insert(p->idx.end(), lb.begin(), lb.end());
         p->nlist_a = (int32_t)la.size();
         p->nlist_b = (int32_t)lb.size();
+        // k_raht_few: so many CTAs a group that a phase's groups fill the device
+        {
+            const int32_t few_a = p->nfew[kSegLong] + p->nfew[kSegMid] + p->nfew[kSegMid2] + p->nfew[kSegRest];
+            auto parts_of = [&](int32_t k) { return k > 0 ? std::min(kFewParts, std::max(1, kFewCtasPerSm * sm_count() / k)) : 1; };
+            p->few_parts_a = parts_of(few_a);
+            p->few_parts_b = parts_of(p->nfew[kSegB]);
+        }
+        // the launch of a group
+        auto seg_of = [&](int gi) {
+            int end = p->ngroups_a_long;
+            if (gi < end) return (int)kSegLong;
+            if (gi < (end += p->ngroups_a_mid)) return (int)kSegMid;
+            if (gi < (end += p->ngroups_a_mid2)) return (int)kSegMid2;
+            return gi < p->ngroups_a ? (int)kSegRest : (int)kSegB;
+        };
         // coefficient regions: a group of k_raht_group shares one frame-interleaved
         // region (stride 32), every other slice owns contiguous planes
         // (window groups first; a region holds the largest slice of its group)
@@ -590,19 +605,25 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         };
         uint64_t c = 0;
         p->coef_win_floats = 0;
-        uint64_t few_max = 1;  // points of a small group's slices
-        uint32_t wide_max = 1;  // of a slice of another group
+        for (uint64_t& f : p->few_floats) f = 0;
+        uint32_t wide_max = 1;  // points of a slice of k_raht_group's
         for (int32_t gi = 0; gi < p->ngroups_a + p->ngroups_b; ++gi) {
             const GroupDesc& g = p->groups[gi];
             if (is_small(gi)) {
+                uint64_t gn = 1;
                 for (int l = 0; l < g.count; ++l) {
                     SliceWork& w = W[p->idx[g.first + l]];
                     w.coef_off = c;
                     w.coef_stride = 1;
                     w.coef_lane = 0;
                     c += 3ull * w.n;
-                    few_max = std::max(few_max, (uint64_t)g.count * w.n);
+                    gn = std::max<uint64_t>(gn, w.n);
                 }
+                // a part's two level buffers: its range of every slice's last
+                // internal level (never wider than the leaves), or one whole level
+                const int seg = seg_of(gi);
+                const uint64_t parts = (uint64_t)(seg == kSegB ? p->few_parts_b : p->few_parts_a);
+                p->few_floats[seg] = std::max(p->few_floats[seg], 6 * std::max(gn, g.count * ((gn + parts - 1) / parts)));
                 continue;
             }
             c = align_up(c, 32);  // a region's rows are whole 128-byte lines (vector stores, prefetches)
@@ -628,7 +649,6 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         coef = c;
         p->coef_floats = coef;
         p->grp_floats = 2ull * wide_max * 96;
-        p->few_floats = 6ull * few_max;
         // the prefix of the planes that the long-slice RLGR launch writes
         // (its groups come first; a long slice outside a group extends it)
         p->coef_long_floats = 0;
@@ -653,35 +673,32 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
     off = align_up(off + 4ull * n, 256);
     p->ws_fstatus = off;
     off = align_up(off + 4ull * n, 256);
-    // group kernel: per persistent CTA two level buffers of [width][32 lanes][3]
-    // floats; an internal level of a valid tree is never wider than its leaves
+    // Level buffers, per CTA: k_raht_group two of [width][32 lanes][3] floats (an
+    // internal level of a valid tree is never wider than its leaves), k_raht_few its
+    // part's.  A segment's two launches follow one another on one stream and share a
+    // region; so do phase B's and the rest of phase A's.
     {
         const int32_t* nf = p->nfew;
-        const int32_t few_a = nf[kSegLong] + nf[kSegMid] + nf[kSegMid2] + nf[kSegRest];
-        const int32_t nwide = p->ngroups_a + p->ngroups_b - few_a - nf[kSegB];
+        const int32_t nwide = p->ngroups_a + p->ngroups_b - nf[kSegLong] - nf[kSegMid] - nf[kSegMid2] - nf[kSegRest] - nf[kSegB];
         p->grp_ctas = std::min<int32_t>(nwide, p->tune.group_ctas_per_sm * sm_count());
-        p->ws_grp = off;
-        off = align_up(off + 4ull * p->grp_floats * std::max(p->grp_ctas, 1), 256);
-        // the long-slice groups run beside the others, with level buffers of their own
         p->grp_ctas_long = std::min<int32_t>(p->ngroups_a_long - nf[kSegLong], p->grp_ctas);
-        p->ws_grp_long = off;
-        off = align_up(off + 4ull * p->grp_floats * p->grp_ctas_long, 256);
         p->grp_ctas_mid = std::min<int32_t>(p->ngroups_a_mid - nf[kSegMid], p->grp_ctas);
-        p->ws_grp_mid = off;
-        off = align_up(off + 4ull * p->grp_floats * p->grp_ctas_mid, 256);
         p->grp_ctas_mid2 = p->ngroups_a_mid2 > 0 ? std::min<int32_t>(p->ngroups_a_mid2, p->grp_ctas) : 0;
-        p->ws_grp_mid2 = off;
-        off = align_up(off + 4ull * p->grp_floats * p->grp_ctas_mid2, 256);
-        // the small groups' level buffers: per CTA two of [slice][node][yuv]
-        const int32_t slots = kFewCtasPerSm * sm_count();
-        auto parts_of = [&](int32_t n) { return n > 0 ? std::min(kFewParts, std::max(1, slots / n)) : 1; };
-        p->few_parts_a = parts_of(few_a);
-        p->few_parts_b = parts_of(nf[kSegB]);
+        uint64_t few[kSegs];
         for (int i = 0; i < kSegs; ++i) {
-            p->few_ctas[i] = std::min<int32_t>(nf[i] * (i == kSegB ? p->few_parts_b : p->few_parts_a), slots);
-            p->ws_few[i] = off;
-            off = align_up(off + 4ull * p->few_floats * p->few_ctas[i], 256);
+            p->few_ctas[i] = std::min<int32_t>(nf[i] * (i == kSegB ? p->few_parts_b : p->few_parts_a), kFewCtasPerSm * sm_count());
+            few[i] = p->few_floats[i] * p->few_ctas[i];
         }
+        auto region = [&](int32_t ctas, uint64_t few_floats) {
+            const uint64_t at = off;
+            off = align_up(off + 4ull * std::max(p->grp_floats * ctas, few_floats), 256);
+            return at;
+        };
+        p->ws_grp = p->ws_few[kSegRest] = p->ws_few[kSegB] =
+            region(std::max(p->grp_ctas, 1), std::max(few[kSegRest], few[kSegB]));
+        p->ws_grp_long = p->ws_few[kSegLong] = region(p->grp_ctas_long, few[kSegLong]);
+        p->ws_grp_mid = p->ws_few[kSegMid] = region(p->grp_ctas_mid, few[kSegMid]);
+        p->ws_grp_mid2 = p->ws_few[kSegMid2] = region(p->grp_ctas_mid2, few[kSegMid2]);
         p->ws_counter = off;
         off = align_up(off + 64, 256);
     }
@@ -744,7 +761,7 @@ int run_decode(const pvvc_plan* p, pvvc_state* st, const uint8_t* payload, float
         return launch_raht_group(dw, dg + first, wide, di, st->v, coef, ts, rs, fs, xyz, rgb, p24, status, scratch,
                                  p->grp_floats, ctas, cnt + 2 * seg, on) == cudaSuccess &&
                launch_raht_few(dw, dg + first + wide, few, seg == kSegB ? p->few_parts_b : p->few_parts_a, di, st->v, coef, ts,
-                               rs, fs, xyz, rgb, p24, status, reinterpret_cast<float*>(w + p->ws_few[seg]), p->few_floats,
+                               rs, fs, xyz, rgb, p24, status, reinterpret_cast<float*>(w + p->ws_few[seg]), p->few_floats[seg],
                                p->few_ctas[seg], cnt + 2 * seg + 1, on) == cudaSuccess;
     };
     // every phase-A group, on the main stream

@@ -163,7 +163,7 @@ struct pvvc_plan {
     bool wide_only = false;  // no such split (set before the build)
     int32_t nfew[kSegs] = {}, few_ctas[kSegs] = {};
     int32_t few_parts_a = 1, few_parts_b = 1;
-    uint64_t ws_few[kSegs] = {}, few_floats = 0;  // their level buffers
+    uint64_t ws_few[kSegs] = {}, few_floats[kSegs] = {};  // their level buffers; a CTA's share
     uint64_t coef_floats = 0;
     uint64_t coef_long_floats = 0;  // planes prefix the long-slice RLGR launch writes
     uint64_t coef_mid_floats = 0;   // ... and the medium tier

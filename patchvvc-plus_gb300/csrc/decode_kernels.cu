@@ -1512,8 +1512,11 @@ __global__ void __launch_bounds__(32 * kGrpWarps, 3) k_raht_group(const SliceWor
 // while it goes through (some of) the slices, whose planes are contiguous: the
 // lanes are as full as the level is wide, where k_raht_group's lane per slice
 // leaves 32 - count of them idle, and there are 3 n floats a slice to clear
-// instead of 96 n a group.  The level signal is [slice][node][yuv] in the CTA's
-// scratch region.  The leaves of 32 nodes are contiguous: their colours go
+// instead of 96 n a group.  The level signal of the part's own nodes is
+// [slice][node][yuv] in the CTA's scratch region; a node's children that belong to
+// another part are not kept.  A part's range of a level is no wider than its range
+// of the last one unless empty nodes lie between, and then the slices go through
+// in chunks that fit.  The leaves of 32 nodes are contiguous: their colours go
 // through the warp's shared rows, then a lane writes a point.  At the last
 // internal level the intra slice, when the group has one, goes first: the others
 // read its colours.
@@ -1642,15 +1645,6 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                         emit_leaf(s_mv[f], s_out[f], N < 10, st, lb, 0, cy[0], cy[N], cy[2ull * N], !(fi && f == 0), o);
                     }
             } else {
-                float *gA = bufA, *gB = bufB;
-                const size_t row = 3ull * N;  // a slice's level signal
-                if (tid < na) {
-                    const float* cy = coef + s_coef[tid];
-                    float* g = gA + tid * row;
-                    g[0] = cy[0];
-                    g[1] = cy[N];
-                    g[2] = cy[2ull * N];
-                }
                 if (wid < 2) {
                     // this part's range of each level, upwards: warp 0 its first
                     // node, warp 1 its last one (child offsets ascend: a node's
@@ -1673,10 +1667,19 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                     }
                 }
                 __syncthreads();
-                // this part's nodes of level l of the slices [f0, f0 + nf)
-                auto nodes = [&](int l, int f0, int nf, bool predict) {
+                auto width = [&](int l) { return max(s_hi[l], s_lo[l]) - s_lo[l]; };
+                uint32_t widest = 0;
+                for (int l = 0; l < H - 1; ++l) widest = max(widest, width(l));
+                const size_t row = 3ull * widest;  // a slice's level signal
+                // slices at a time: all, but for a range widened by empty nodes (the
+                // buffers hold a slice of any width up to N, the widest level)
+                const int chunk = widest ? (int)min((uint64_t)na, scratch_floats / 2 / row) : 0;
+                float *gA, *gB;
+                // this part's nodes of level l of the slices [f0, f0 + nf) of a chunk
+                auto nodes = [&](int l, int first, int f0, int nf, bool predict) {
                     const bool last = l == H - 2;
-                    const uint32_t lo = s_lo[l], nj = max(s_hi[l], lo) - lo, nbatch = (nj + 31) / 32;
+                    const uint32_t lo = s_lo[l], nj = width(l), nbatch = (nj + 31) / 32;
+                    const uint32_t clo = last ? 0u : s_lo[l + 1], cnj = last ? 0u : width(l + 1);
                     // the slices in chunks, so that every warp has two units or more
                     const int chunks = nbatch ? min(nf, (int)((2 * kFewWarps + nbatch - 1) / nbatch)) : 1;
                     const int per = (nf + chunks - 1) / max(chunks, 1);
@@ -1695,18 +1698,21 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                         const uint32_t base = __shfl_sync(0xffffffffu, rec.cb, 0);
                         const uint32_t total = __shfl_sync(0xffffffffu, rec.cb + __popc(rec.byte), nv - 1) - base;
                         for (int f = fa; f < fb; ++f) {
-                            const float* g = gA + f * row + 3ull * j;
+                            const float* g = gA + (f - first) * row + 3ull * (j - lo);
                             float oy[8], ou[8], ov[8];
                             lane_inverse(rec, coef + s_coef[f], N, g[0], g[1], g[2], oy, ou, ov);
                             if (!last) {
-                                float* gb = gB + f * row + 3ull * rec.cb;
+                                float* const gb = gB + (f - first) * row;
+                                uint32_t at = rec.cb - clo;  // (unsigned: children before the range are beyond it)
 #pragma unroll
                                 for (int c = 0; c < 8; ++c) {
                                     if (!(rec.byte & (0x80u >> c))) continue;
-                                    gb[0] = oy[c];
-                                    gb[1] = ou[c];
-                                    gb[2] = ov[c];
-                                    gb += 3;
+                                    if (at < cnj) {
+                                        gb[3ull * at] = oy[c];
+                                        gb[3ull * at + 1] = ou[c];
+                                        gb[3ull * at + 2] = ov[c];
+                                    }
+                                    ++at;
                                 }
                                 continue;
                             }
@@ -1728,18 +1734,33 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                         }
                     }
                 };
-                for (int l = 0; l < H - 2; ++l) {
-                    nodes(l, 0, na, true);
+                for (int first = 0; chunk && first < na; first += chunk) {
+                    const int nf = min(chunk, na - first);
+                    gA = bufA;
+                    gB = bufB;
+                    if (tid < nf) {
+                        const float* cy = coef + s_coef[first + tid];
+                        float* g = gA + tid * row;
+                        g[0] = cy[0];
+                        g[1] = cy[N];
+                        g[2] = cy[2ull * N];
+                    }
                     __syncthreads();
-                    float* t = gA;
-                    gA = gB;
-                    gB = t;
-                }
-                if (fi) {
-                    nodes(H - 2, 0, 1, false);
+                    for (int l = 0; l < H - 2; ++l) {
+                        nodes(l, first, first, nf, true);
+                        __syncthreads();
+                        float* t = gA;
+                        gA = gB;
+                        gB = t;
+                    }
+                    const int f1 = first == 0 ? fi : 0;
+                    if (f1) {
+                        nodes(H - 2, 0, 0, 1, false);
+                        __syncthreads();
+                    }
+                    nodes(H - 2, first, first + f1, nf - f1, true);
                     __syncthreads();
                 }
-                nodes(H - 2, fi, na - fi, true);
             }
         }
         __syncthreads();

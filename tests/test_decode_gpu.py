@@ -639,3 +639,43 @@ def test_tree_wider_than_its_leaves_is_malformed(pvvc_lib, oracle, torch, nframe
                 assert np.array_equal(xyz[a + at:a + at + n].view(np.uint32), ox[at:at + n].view(np.uint32))
                 assert rgb_matches(rgb[a + at:a + at + n], orgb[at:at + n], yuv).all()
             at += n
+
+
+# node 0 and node 63 of a level of 64 have children: a part of the last internal
+# level with children of both has 64 ancestors, more than its range
+_SPARSE = [[0xFF], [0xFF] * 8, [0xFE] + [0] * 62 + [0xFF], [0xFF] * 15]
+
+
+@pytest.mark.parametrize("nframes", [1, 2, 8, 30, 33])
+def test_sparse_levels_in_parts(pvvc_lib, oracle, torch, nframes):
+    """A group over several CTAs whose ranges of the upper levels are wider than of
+    the last one: every frame equals the oracle's."""
+    frames = _crafted_frames(pvvc_lib, oracle, [_SPARSE, _FULL], nframes)
+    batch = pvvc_lib.pack_frames(frames)
+    dec = pvvc_lib.Decoder(nslots=2, max_leaves=4096)
+    decs = [oracle.decoder() for _ in range(2)]
+    xyz, rgb, st = decode_batch(torch, pvvc_lib, dec, batch)
+    assert (st == 0).all()
+    for f, fr in enumerate(frames):
+        a, b = batch.frame_first_point[f], batch.frame_first_point[f + 1]
+        ox, orgb, ost = oracle.decode_frame(decs, fr, nthreads=1)
+        yuv = np.concatenate([d.get_patch()[1] for d in decs])
+        assert (ost == 0).all() and np.array_equal(xyz[a:b].view(np.uint32), ox.view(np.uint32)), f
+        assert rgb_matches(rgb[a:b], orgb, yuv).all(), f
+
+
+@pytest.mark.parametrize("patches,nframes,points", [(1, 1, 300000), (1, 2, 300000), (1, 30, 300000), (1, 32, 5000),
+                                                    (8, 8, 20000), (59, 30, 8000), (100, 17, 3000), (400, 2, 2000)])
+def test_workspace_of_few_large_groups(pvvc_lib, patches, nframes, points):
+    """A group's workspace does not grow with the CTAs it is spread over: at most
+    the planes of 32 lanes, one pair of level buffers of 32 lanes, and a level
+    pair a slice (1152 + 24 nframes bytes a point of the patch)."""
+    n = patches * nframes
+    z8, z4 = np.zeros(n, np.uint64), np.zeros(n, np.uint32)
+    f = np.repeat(np.arange(nframes), patches)
+    b = pvvc_lib.Batch(np.zeros(64, np.uint8), np.tile(np.arange(patches, dtype=np.int32), nframes),
+                       np.where(f == 0, 1, 3).astype(np.uint8), np.full(n, points, np.uint32), np.full(n, 8, np.uint8),
+                       np.zeros((n, 16), np.float32), z8, z4, z8, z4, z8, np.zeros(nframes + 1, np.int64),
+                       np.zeros(nframes + 1, np.int64))
+    ws = pvvc_lib.Plan(b).workspace_bytes
+    assert ws <= patches * points * (1152 + 24 * nframes) + (1 << 20), (ws, ws / (patches * points))
