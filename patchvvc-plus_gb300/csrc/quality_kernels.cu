@@ -278,6 +278,7 @@ __global__ void __launch_bounds__(kQThreads) k_q_query(QPair pr, double* __restr
         float best = FLT_MAX;
         int bi = 0x7FFFFFFF;
         auto run = [&](uint32_t row, int x0, int x1) {  // the points of cells [x0, x1] of a row
+            if (x0 > x1) return;
             const uint32_t e = __ldg(cell + row + x1 + 1);
             for (uint32_t k = __ldg(cell + row + x0); k < e; ++k) {
                 const float4 p = __ldg(sorted + k);
@@ -301,9 +302,12 @@ __global__ void __launch_bounds__(kQThreads) k_q_query(QPair pr, double* __restr
             return fmaxf(d - pad, 0.f);
         };
         // a first point from the query's own cell, or boxes of growing size; then
-        // the rows of cells inside the ball to the best one
-        const int cx = qcell(g, x, 0), cy = qcell(g, y, 1), cz = qcell(g, z, 2);
-        run(((uint32_t)cz * g.dim[1] + cy) * g.dim[0], cx, cx);
+        // the rows of cells inside the ball to the best one.  The box before, [ax0,
+        // ax1] and so on, is done with: a far outlier makes cells of very many
+        // points, which cost twice as much when each was gone through again (200k
+        // points in one cell: 99 ms, 48 now).
+        int ax0 = qcell(g, x, 0), ay0 = qcell(g, y, 1), az0 = qcell(g, z, 2), ax1 = ax0, ay1 = ay0, az1 = az0;
+        run(((uint32_t)az0 * g.dim[1] + ay0) * g.dim[0], ax0, ax0);
         float rad = 0.5f * g.h;
         for (bool last = false; !last; rad *= 4.f) {
             const bool bounded = bi != 0x7FFFFFFF;
@@ -319,9 +323,13 @@ __global__ void __launch_bounds__(kQThreads) k_q_query(QPair pr, double* __restr
                 for (int yy = y0; yy <= y1; ++yy) {
                     const float gy = gap(yy, y, 1);
                     if (gz2 + gy * gy * 0.9999f > best) continue;
-                    run(((uint32_t)zz * g.dim[1] + yy) * g.dim[0], x0, x1);
+                    const uint32_t row = ((uint32_t)zz * g.dim[1] + yy) * g.dim[0];
+                    const bool in = zz >= az0 && zz <= az1 && yy >= ay0 && yy <= ay1;
+                    run(row, x0, in ? min(x1, ax0 - 1) : x1);
+                    if (in) run(row, max(x0, ax1 + 1), x1);
                 }
             }
+            ax0 = x0, ax1 = x1, ay0 = y0, ay1 = y1, az0 = z0, az1 = z1;
         }
         float qc[3], tc[3];
         yuv601(c.rgb + 3ull * i, qc);

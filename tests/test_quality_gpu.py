@@ -88,3 +88,26 @@ def test_quality_block_edges(q, na, nb):
     want = np.stack([side(a, ac, b, bc), side(b, bc, a, ac)], 1).reshape(-1)
     # the float YUV is off by at most 3 roundings of values below 512
     assert np.allclose(q.mse(a, ac, b, bc), want, rtol=1e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("na,nb,far", [(300, 300, 40.0), (300, 5000, 1e4), (5000, 300, 1e6), (2000, 2000, 100.0)])
+def test_quality_crowded_cells(q, na, nb, far):
+    """Clouds with a point far off, so that the others share one cell or a few of
+    them, against brute force (as above)."""
+    rng = np.random.default_rng(na + nb)
+    a = rng.integers(0, 20, (na, 3)).astype(np.float32)
+    b = rng.integers(0, 20, (nb, 3)).astype(np.float32) + np.float32(0.5)
+    a[0] += np.float32(far)
+    b[0] += np.float32(far)
+    ac = rng.integers(0, 256, (na, 3)).astype(np.uint8)
+    bc = rng.integers(0, 256, (nb, 3)).astype(np.uint8)
+    K = np.array([[0.299, 0.587, 0.114], [-0.168736, -0.331264, 0.5], [0.5, -0.418688, -0.081312]])
+
+    def side(p, pc, t, tc):
+        d = ((p[:, None].astype(np.float64) - t[None]) ** 2).sum(2)
+        j = d.argmin(1)
+        e = (pc.astype(np.float64) - tc[j]) @ K.T
+        return [d.min(1).mean()] + list((e * e).mean(0))
+
+    want = np.stack([side(a, ac, b, bc), side(b, bc, a, ac)], 1).reshape(-1)
+    assert np.allclose(q.mse(a, ac, b, bc), want, rtol=1e-5, atol=1e-4)
