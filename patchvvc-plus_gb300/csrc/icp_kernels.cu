@@ -65,7 +65,10 @@ struct GridHdr {  // per pair
     float h;
     int dim[3];
     float eps;  // bounds how far rounding can put a point outside its cell's box
+    int crowded;  // one cell holds most of the points (a far outlier leaves the others there)
 };
+// (patches without one have up to a quarter of their points in a cell)
+__device__ __forceinline__ bool crowds(int count, uint32_t n) { return count > 64 && (uint32_t)count > n / 2; }
 
 // ---------------------------------------------------------------------------
 template <int T>
@@ -162,6 +165,7 @@ __global__ void __launch_bounds__(T) k_grid(const float* __restrict__ pts, const
         s_box[3] = g.h;
         s_box[4] = __int_as_float(g.dim[0]);
         s_box[5] = __int_as_float(g.dim[1] * 1024 + g.dim[2]);
+        g.crowded = 0;  // (below)
         g.eps = 0.f;
         for (int k = 0; k < 3; ++k) g.eps = fmaxf(g.eps, 1e-6f * (fabsf(g.lo[k]) + e[k]));
         hdr[pair] = g;
@@ -184,9 +188,13 @@ __global__ void __launch_bounds__(T) k_grid(const float* __restrict__ pts, const
     // exclusive scan of C+1 counters (serial per warp chunk, then warp offsets)
     const int per = (C + 1 + T - 1) / T;
     int loc = 0;
+    bool crowded = false;
     for (int k = 0; k < per; ++k) {
         const int c = tid * per + k;
-        if (c <= C) loc += s_cnt[c];
+        if (c <= C) {
+            loc += s_cnt[c];
+            crowded |= crowds(s_cnt[c], n);
+        }
     }
     int x = loc;
     for (int o = 1; o < 32; o <<= 1) {
@@ -206,7 +214,8 @@ __global__ void __launch_bounds__(T) k_grid(const float* __restrict__ pts, const
             s_cnt[c] = run;  // inclusive prefix of counts[0..c] == start of cell c (counts shifted by one)
         }
     }
-    __syncthreads();
+    crowded = __syncthreads_or(crowded);
+    if (tid == 0) hdr[pair].crowded = crowded;
     int* cs = cstart + cell_base(kmul, a, pair);
     for (int c = tid; c <= C; c += T) cs[c] = s_cnt[c];
     __syncthreads();
@@ -231,6 +240,10 @@ __global__ void __launch_bounds__(T) k_grid(const float* __restrict__ pts, const
 // cell of an axis is open upwards (it also holds what a clamped axis leaves
 // over), and squared bounds keep a margin of 1e-4, so no point that could win
 // is skipped.
+//
+// EARLY: a ball that lies within the rings is done, and the cells' points are not
+// gone through a second time.  Cells of many points need that (900 points in one
+// cell: a search costs half as much); elsewhere the ball hardly ever lies so.
 struct NearPoint {
     float d;       // squared distance; FLT_MAX: none
     int j;         // into sp; -1: none
@@ -244,6 +257,7 @@ __device__ __forceinline__ float dist2(const float4& p, float qx, float qy, floa
     const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
     return dx * dx + dy * dy + dz * dz;
 }
+template <bool EARLY>
 __device__ __forceinline__ NearPoint grid_nn(const GridHdr& g, const int* __restrict__ cs, const float4* __restrict__ sp,
                                              float qx, float qy, float qz, int start) {
     NearPoint r{FLT_MAX, -1};
@@ -260,11 +274,13 @@ __device__ __forceinline__ NearPoint grid_nn(const GridHdr& g, const int* __rest
     };
     const float inv = 1.0f / g.h;
     auto cell = [&](float v, int k) { return min(max((int)floorf((v - g.lo[k]) * inv), 0), g.dim[k] - 1); };
+    const float pad = 0.001f * g.h + g.eps;  // of the cell indices' rounding
     if (start >= 0) visit(start);
     if (r.j < 0) {
         const int cx = cell(qx, 0), cy = cell(qy, 1), cz = cell(qz, 2);
         const int maxr = max(g.dim[0], max(g.dim[1], g.dim[2]));
-        for (int t = 0; t <= maxr && r.j < 0; ++t)
+        int t = 0;
+        for (; t <= maxr && r.j < 0; ++t)
             for (int z = max(cz - t, 0); z <= min(cz + t, g.dim[2] - 1); ++z)
                 for (int y = max(cy - t, 0); y <= min(cy + t, g.dim[1] - 1); ++y) {
                     const int row = (z * g.dim[1] + y) * g.dim[0];
@@ -281,6 +297,12 @@ __device__ __forceinline__ NearPoint grid_nn(const GridHdr& g, const int* __rest
                     }
                 }
         if (r.j < 0) return r;
+        if (EARLY) {
+            const float o = (sqrt_fast(r.d) * 1.0001f + g.eps) * 1.0001f + pad;
+            if (cell(qx - o, 0) > cx - t && cell(qx + o, 0) < cx + t && cell(qy - o, 1) > cy - t && cell(qy + o, 1) < cy + t &&
+                cell(qz - o, 2) > cz - t && cell(qz + o, 2) < cz + t)
+                return r;
+        }
     }
     // the ball to the best point
     float at = r.d, rad = sqrt_fast(r.d) * 1.0001f + g.eps;
@@ -290,7 +312,6 @@ __device__ __forceinline__ NearPoint grid_nn(const GridHdr& g, const int* __rest
         const float d = q < a ? a - q : (q > a + g.h && c < g.dim[k] - 1 ? q - (a + g.h) : 0.f);
         return fmaxf(d - g.eps, 0.f);
     };
-    const float pad = 0.001f * g.h + g.eps;  // of the cell indices' rounding
     const int z1 = cell(qz + rad0 + pad, 2), y0 = cell(qy - rad0 - pad, 1), y1 = cell(qy + rad0 + pad, 1);
     for (int z = cell(qz - rad0 - pad, 2); z <= z1; ++z) {
         const float gz = gap(z, qz, 2), gz2 = gz * gz;
@@ -506,8 +527,14 @@ __device__ __forceinline__ int icp_class(uint32_t n) {  // 0: 5,793 points or mo
     return min(max(25 - (31 - __clz((int)(m * m | 1u))), 0), kIcpClasses - 1);  // floor(2 log2 n)
 }
 
-template <bool KEEP, int T>
-__global__ void __launch_bounds__(T, 1024 / T) k_icp(const float* __restrict__ src, const uint32_t* __restrict__ soff,
+//
+// Without KEEP, pairs whose target is crowded have a launch of their own (CROWDED;
+// a CTA of the other kind's pair returns): in one kernel the early end of their
+// searches costs the others 10 to 25% in registers.  16 pairs with a far outlier
+// each, 10 iterations: 25.7 ms with rings and ball over the same cell, 11.5 now; 300
+// of them 165 and 73.
+template <bool KEEP, int T, bool CROWDED = KEEP>
+__global__ void __launch_bounds__(T, !KEEP && CROWDED ? 2 : 1024 / T) k_icp(const float* __restrict__ src, const uint32_t* __restrict__ soff,
                                                      const uint32_t* __restrict__ toff, const GridHdr* __restrict__ hdr,
                                                      const int* __restrict__ cstart, const float4* __restrict__ tsorted,
                                                      const float* __restrict__ init, pvvc_icp_params prm,
@@ -524,6 +551,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_icp(const float* __restrict__ s
     if (gridDim.y > 1 && icp_class(b - a) != (int)blockIdx.y) return;
     const uint32_t tb = toff[pair];
     if (toff[pair + 1] > cap || tb > toff[pair + 1]) {  // k_grid built no grid for this pair
+        if (!KEEP && CROWDED) return;  // (the other launch's)
         if (tid < 16) T_out[pair * 16 + tid] = __int_as_float(0x7fc00000);
         if (tid == 0) {
             if (mse_out) mse_out[pair] = __int_as_float(0x7fc00000);
@@ -532,6 +560,7 @@ __global__ void __launch_bounds__(T, 1024 / T) k_icp(const float* __restrict__ s
         }
         return;
     }
+    if (!KEEP && (hdr[pair].crowded != 0) != CROWDED) return;
     const GridHdr g = hdr[pair];
     const int* const cs = cstart + cell_base(kIcpCellMul, tb, pair);
     const float4* const sp = tsorted + tb;
@@ -557,13 +586,13 @@ __global__ void __launch_bounds__(T, 1024 / T) k_icp(const float* __restrict__ s
         for (uint32_t i = a + tid; i < b; i += T) {
             float qx, qy, qz;
             moved(i, qx, qy, qz);
-            near_j[i] = grid_nn(g, cs, sp, qx, qy, qz, first ? -1 : near_j[i]).j;
+            near_j[i] = grid_nn<CROWDED>(g, cs, sp, qx, qy, qz, first ? -1 : near_j[i]).j;
         }
         if (T > kIcpThreads) __syncthreads();  // (else a thread sums the points it searched)
     };
     // source point i's nearest target point, and its squared distance
     auto nearest = [&](uint32_t i, float qx, float qy, float qz, float4& m) -> float {
-        const int j = keep ? near_j[i] : grid_nn(g, cs, sp, qx, qy, qz, -1).j;
+        const int j = keep ? near_j[i] : grid_nn<CROWDED>(g, cs, sp, qx, qy, qz, -1).j;
         m = j >= 0 ? __ldg(sp + j) : make_float4(0.f, 0.f, 0.f, 0.f);
         return j >= 0 ? dist2(m, qx, qy, qz) : FLT_MAX;
     };
@@ -705,7 +734,7 @@ __global__ void __launch_bounds__(kIcpThreads) k_nn_mean(const float* __restrict
         const float qx = M[0] * x + M[1] * y + M[2] * z + M[3];
         const float qy = M[4] * x + M[5] * y + M[6] * z + M[7];
         const float qz = M[8] * x + M[9] * y + M[10] * z + M[11];
-        acc.add(grid_nn(g, cs, sorted + gb, qx, qy, qz, -1).d);
+        acc.add(grid_nn<true>(g, cs, sorted + gb, qx, qy, qz, -1).d);
     }
     double v = acc.value();
     for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -1174,7 +1203,10 @@ extern "C" int pvvc_icp_batch_noalloc(int32_t npairs, const float* src_xyz, cons
     void* ia[] = {(void*)&src_xyz, (void*)&src_off, (void*)&tgt_off, (void*)&chdr, (void*)&ccs, (void*)&csorted,
                   (void*)&init, (void*)&prm, (void*)&T_out, (void*)&mse_out, (void*)&iters_out,
                   (void*)&converged_out, (void*)&cap, (void*)&no_j, (void*)&no_src};
-    if (cudaLaunchKernel((const void*)k_icp<false, kIcpThreads>, icp_grid(npairs), dim3(kIcpThreads), ia, 0, s) != cudaSuccess)
+    if (cudaLaunchKernel((const void*)k_icp<false, kIcpThreads, false>, icp_grid(npairs), dim3(kIcpThreads), ia, 0, s) !=
+            cudaSuccess ||
+        cudaLaunchKernel((const void*)k_icp<false, kIcpThreads, true>, icp_grid(npairs), dim3(kIcpThreads), ia, 0, s) !=
+            cudaSuccess)
         return PVVC_ERR_CUDA;
     return PVVC_OK;
 }

@@ -216,3 +216,55 @@ def test_gpu_icp_flat_patches(pvvc_lib, oracle, flat):
     assert rotation_error_deg(T, np.array([To]))[0] < ROT_TOL_DEG
     assert _trans_err(T, np.array([To]), p)[0] < TRANS_TOL_VOX
     assert abs(mse[0] - fit) <= MSE_RTOL * fit + 1e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("far", [30.0, 1e3, 1e6])
+def test_gpu_icp_far_outliers(pvvc_lib, far):
+    """Clouds with a point far off, which leaves the others in one or a few cells of
+    the grid, between pairs without one: ICP with and without kept neighbours gives
+    the same bits, each pair those it has alone, and the clouds' MSE is brute
+    force's."""
+    import ctypes as C
+    import torch
+    from pvvc import _lib as L
+    from pvvc.icp import IcpBatch, Pairs
+    rng = np.random.default_rng(6)
+    src, tgt = [], []
+    for i, n in enumerate((40, 66, 300, 700, 1500, 900)):
+        s = rng.integers(0, 30, (n, 3)).astype(np.float32)
+        t = (s + rng.normal(0, 0.4, s.shape)).astype(np.float32)
+        if i != 3:
+            t[-1] += np.float32(far)
+            s[0] += np.float32(far if i % 2 else 0)
+        src.append(s)
+        tgt.append(t)
+
+    def noalloc(b, iters):
+        prm = L.IcpParams(1e6, iters, 0.0, 0.0, 1e-6)
+        L.check(L.lib().pvvc_icp_batch_noalloc(b.n, b.src.data_ptr(), b.soff.data_ptr(), b.tgt.data_ptr(), b.toff.data_ptr(),
+                                               None, C.byref(prm), b.T.data_ptr(), b.mse.data_ptr(), b.iters.data_ptr(),
+                                               b.conv.data_ptr(), b.nt, torch.cuda.current_stream().cuda_stream), "noalloc")
+
+    def batch(ids):
+        return IcpBatch(Pairs([src[i] for i in ids], [tgt[i] for i in ids], np.tile(np.eye(4), (len(ids), 1, 1))))
+
+    b = batch(range(6))
+    b.run(max_iter=8)
+    want = b.results()
+    mse = b.cloud_mse()
+    for v in (b.T, b.mse, b.iters, b.conv):
+        v.zero_()
+    noalloc(b, 8)
+    for g, w in zip(b.results(), want):
+        assert np.array_equal(g, w)
+    for i in range(6):
+        one = batch([i])
+        noalloc(one, 8)
+        for g, w in zip(one.results(), want):
+            assert np.array_equal(g[0], w[i])
+        m = (src[i].astype(np.float64) @ want[0][i, :3, :3].astype(np.float64).T + want[0][i, :3, 3]).astype(np.float32)
+        d = ((m[:, None].astype(np.float64) - tgt[i][None]) ** 2).sum(2)
+        # float32 coordinates of the size of `far`
+        tol = 1e-5 * max(d.min(1).mean(), d.min(0).mean()) + 1e-5 + (4e-7 * far) ** 2 + 1e-6 * far
+        assert abs(mse[i] - max(d.min(1).mean(), d.min(0).mean())) <= tol, i
