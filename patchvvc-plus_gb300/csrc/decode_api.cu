@@ -518,7 +518,12 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 if (p->ngroups_a_long > 0 && p->side.ensure(true) != cudaSuccess) return PVVC_ERR_CUDA;
                 if (p->ngroups_a_mid > 0 && p->side2.ensure() != cudaSuccess) return PVVC_ERR_CUDA;
                 if (p->ngroups_a_mid2 > 0 && p->side3.ensure() != cudaSuccess) return PVVC_ERR_CUDA;
-                p->nfew[kSegLong] = p->ngroups_a_long;  // decoded into planes of their own, as small groups are
+                // the long tier by k_raht_few too (and decoded into planes of its own,
+                // as small groups are), but for large batches of full groups
+                int32_t long_slices = 0;
+                for (int gi = 0; gi < p->ngroups_a_long; ++gi) long_slices += gw[gi].count;
+                const bool long_wide = nw >= kLongWidePerSm * sm_count() && long_slices >= kLongWideCount * p->ngroups_a_long;
+                p->nfew[kSegLong] = long_wide ? 0 : p->ngroups_a_long;
                 p->nfew[kSegMid] = p->nfew[kSegMid2] = 0;
                 p->nfew[kSegRest] = few_last(gr);
                 ga = gw;
@@ -601,7 +606,7 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
         // region (stride 32), every other slice owns contiguous planes
         // (window groups first; a region holds the largest slice of its group)
         auto is_small = [&](int gi) {
-            return is_few(p->groups[gi]) || (p->nwin > 0 && gi < p->ngroups_a_long);
+            return is_few(p->groups[gi]) || (p->nwin > 0 && gi < p->nfew[kSegLong]);
         };
         uint64_t c = 0;
         p->coef_win_floats = 0;

@@ -24,10 +24,19 @@ constexpr int kRlgrLongBlock = 128;
 // the long tier takes kWinGroupsPerLongCta of them per long CTA.
 constexpr int kWinGroupMin = 16;
 constexpr int kWinGroupsPerLongCta = 4;
-// In a batch with window groups, groups of fewer slices (and the long tier's)
-// are inverse-transformed by k_raht_few, the others by k_raht_group; in any other
-// batch all by k_raht_few.
+// In a batch with window groups, groups of fewer slices are inverse-transformed
+// by k_raht_few, the others by k_raht_group; in any other batch all by k_raht_few.
 constexpr int kFewBelow = 16;
+// The long tier's groups go to k_raht_few as well, whatever their size: it splits
+// each over several CTAs, a shorter tail for more instructions a point.  That pays
+// while the other groups do not fill the device beside it, below kLongWidePerSm
+// window groups per SM, or while lanes would idle in k_raht_group, below
+// kLongWideCount slices a group.  GoPs of 30 frames and 470 groups at once, few /
+// group, ms: one 1.19 / 1.76, two 1.70 / 1.85, four 2.51 / 2.67; six 3.65 / 3.53, ten
+// 5.57 / 5.51, and at steps of 16 and 32 5.24 / 5.15 and 5.08 / 4.99.  Ten of 17 and 24
+// frames at a step of 32: 4.72 / 4.78 and 4.90 / 4.87.
+constexpr int kLongWidePerSm = 16;
+constexpr int kLongWideCount = 28;
 
 struct SliceWork {
     uint64_t col_off;   // colour payload byte offset

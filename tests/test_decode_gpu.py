@@ -679,3 +679,30 @@ def test_workspace_of_few_large_groups(pvvc_lib, patches, nframes, points):
                        np.zeros(nframes + 1, np.int64))
     ws = pvvc_lib.Plan(b).workspace_bytes
     assert ws <= patches * points * (1152 + 24 * nframes) + (1 << 20), (ws, ws / (patches * points))
+
+
+@pytest.mark.parametrize("nframes", [17, 28])
+def test_long_tier_of_a_large_batch(pvvc_lib, oracle, torch, nframes):
+    """Sixteen window groups an SM: the long tier's groups are inverse-transformed
+    by the group kernel when their frames fill its lanes (28), by the node kernel
+    otherwise (17); the first stream equals the oracle's decode, the others the
+    first."""
+    frames = _large_value_frames(pvvc_lib, nframes)
+    streams = -(-16 * torch.cuda.get_device_properties(0).multi_processor_count // 8)
+    one, batch = _streams(pvvc_lib, frames, streams)
+    # both plans have a long tier, cleared beforehand: 64 groups, in planes of 32
+    # lanes or of their own
+    clear = pvvc_lib.Plan(batch).info()["clear_bytes"]
+    big = int(batch.size.max())
+    assert clear == 64 * 3 * 4 * big * (32 if nframes == 28 else nframes)
+    dec = pvvc_lib.Decoder(nslots=8 * streams, max_leaves=4096)
+    xyz, rgb, st = decode_batch(torch, pvvc_lib, dec, batch)
+    assert (st == 0).all(), np.unique(st)
+    P = xyz.shape[0] // streams
+    for s in range(1, streams):
+        for a in (xyz, rgb):
+            assert np.array_equal(a[s * P:(s + 1) * P].view(np.uint8), a[:P].view(np.uint8)), s
+    for fi, (ox, orgb, ost, yuv) in enumerate(oracle_decode(oracle, pvvc_lib, frames, 16)):
+        a, b = one.frame_first_point[fi], one.frame_first_point[fi + 1]
+        assert np.array_equal(xyz[a:b].view(np.uint32), ox.view(np.uint32)), fi
+        assert rgb_matches(rgb[a:b], orgb, yuv).all(), fi
