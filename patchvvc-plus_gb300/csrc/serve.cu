@@ -337,7 +337,18 @@ int pvvc_server::launch(Batch& b) {
     const uint64_t zstart = align_up(bytes + 16, 16), a_src = align_up(zstart + zbytes, 16), a_dst = a_src + 8ull * nz,
                    a_len = a_dst + 8ull * nz, a_cap = a_len + 4ull * nz, a_slice = a_cap + 4ull * nz,
                    a_stat = a_slice + 4ull * nz, total = nz ? a_stat + 4ull * nz : bytes;
-    if (b.h_payload.ensure(total + 16) != cudaSuccess || b.d_payload.ensure(total + 16) != cudaSuccess ||
+    // device buffers of the reservation: what they grow by is added to it
+    auto grow = [&](DevBuf& d, size_t n) {
+        const size_t was = d.cap;
+        const cudaError_t e = d.ensure(n);
+        if (d.cap != was) {
+            std::lock_guard<std::mutex> g(mu);
+            reserved += d.cap;
+            reserved -= was;
+        }
+        return e;
+    };
+    if (b.h_payload.ensure(total + 16) != cudaSuccess || grow(b.d_payload, total + 16) != cudaSuccess ||
         b.h_status.ensure(4ull * std::max(nsl, 1)) != cudaSuccess || b.d_status.ensure(4ull * std::max(nsl, 1)) != cudaSuccess)
         return PVVC_ERR_NOMEM;
     b.slot.resize(nsl);
@@ -398,7 +409,7 @@ int pvvc_server::launch(Batch& b) {
                       b.gsz.data(), b.coff.data(), b.csz.data(), b.oo.data()};
     int rc = build_plan(&d, &b.plan, &cfg.tune, copy);
     if (rc) return rc;
-    if (b.ws.ensure(b.plan.ws_bytes) != cudaSuccess) return PVVC_ERR_NOMEM;
+    if (grow(b.ws, b.plan.ws_bytes) != cudaSuccess) return PVVC_ERR_NOMEM;
     if (cudaMemcpyAsync(b.d_payload.p, hp, (nz ? total : off) + 16, cudaMemcpyHostToDevice, copy) != cudaSuccess ||
         cudaEventRecord(b.e_h2d, copy) != cudaSuccess || cudaStreamWaitEvent(compute, b.e_h2d, 0) != cudaSuccess ||
         cudaEventRecord(b.e_start, compute) != cudaSuccess)
@@ -499,7 +510,11 @@ extern "C" int pvvc_server_create(const pvvc_server_config* cfg_in, pvvc_server*
     s->cfg = c;
     s->t0 = std::chrono::steady_clock::now();
     if (cudaGetDevice(&s->device) != cudaSuccess || prepare_kernels() != cudaSuccess) return PVVC_ERR_CUDA;
-    // fixed reservations: output ring, per-batch staging and workspace
+    // Fixed reservations: output ring, per-batch staging and workspace.  A
+    // workspace is reserved for batches of small groups, whose level buffers are
+    // at most one 32-lane pair a CTA of the group kernel (k_raht_few's parts hold
+    // no more between them), and 96 bytes a point for everything else; a batch
+    // that needs more has its buffers grown, and the reservation with them.
     const uint64_t ring_bytes = 15ull * c.ring_points;
     const uint64_t grp_scratch = 2ull * c.max_leaves * 96 * 4 * (uint64_t)(c.tune.group_ctas_per_sm * sm_count());
     const uint64_t ws_guess = 96ull * c.max_batch_points + grp_scratch + (1ull << 20);
