@@ -628,6 +628,18 @@ extern "C" int pvvc_fitting_clouds(pvvc_fitter* f, int32_t ngops, const int32_t*
         f->iters.ensure(4 * cells.size()) || f->start.ensure(4 * N) || f->mem.ensure(4 * N) ||
         f->ctl.ensure(sizeof(FitCtl) * cells.size()) || f->side[0].ensure() || f->side[1].ensure())
         return PVVC_ERR_NOMEM;
+    // An error from here on leaves with nothing of the call under way: its copies
+    // read the fitter's host arrays and its launches, on three streams, the device
+    // ones, which the next call fills again.
+    struct Settle {
+        pvvc_fitter* f;
+        cudaStream_t s;
+        ~Settle() {
+            if (!f) return;
+            cudaStreamSynchronize(s);
+            for (SideStream& sd : f->side) cudaStreamSynchronize(sd.s);
+        }
+    } settle{f, s};
     if (cudaMemcpyAsync(f->pts.p, xyz + 3ull * p_first, 12 * N, cudaMemcpyHostToDevice, s) != cudaSuccess ||
         cudaMemcpyAsync(f->d_order.p, f->order.p, 4 * N, cudaMemcpyHostToDevice, s) != cudaSuccess)
         return PVVC_ERR_CUDA;
@@ -747,6 +759,7 @@ extern "C" int pvvc_fitting_clouds(pvvc_fitter* f, int32_t ngops, const int32_t*
     if (cudaMemcpyAsync(out_xyz, f->out.p, 12 * total_out, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return PVVC_ERR_CUDA;
+    settle.f = nullptr;
     if (stats) {
         int64_t it = 0, ex = 0;
         for (size_t c = 0; c < cells.size(); ++c) {
