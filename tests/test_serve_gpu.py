@@ -202,19 +202,21 @@ def test_zstd_frames_served_like_raw(pvvc_lib, torch, sequences):
 
 
 def test_reservation_follows_grown_buffers(pvvc_lib, torch, sequences):
-    """A batch larger than the server was set up for has its buffers grown, and the
-    memory the server reports holding grows with them."""
+    """A batch with more payload than the server was set up for (4 bytes a point of
+    its largest batch) has its buffers grown, and the memory the server reports
+    holding grows with them."""
     from pvvc.serve import slots_needed
     frames = sequences[1]
-    srv = _server(pvvc_lib, max_batch_points=500, inflight=1)
+    f = pvvc_lib.parse_frame(frames[0])
+    f.color = [c + bytes(2000) for c in f.color]  # (bytes after the last symbol are not read)
+    need = sum(len(g) + len(c) for g, c in zip(f.geometry, f.color))
+    staged = 4 * f.points + 4096
+    assert need > staged
+    srv = _server(pvvc_lib, max_batch_points=f.points, inflight=1)
     sid = srv.open_stream(slots_needed(frames))
     before = srv.stats()["reserved_bytes"]
-    payload = len(frames[0])
-    assert payload > 4 * 500 + 4096  # beyond the staging buffer set up
-    srv.submit(sid, frames[0], tag=0)
+    srv.submit(sid, pvvc_lib.write_frame(f), tag=0)
     assert _drain(srv, 1)[0][0] == 0
     after = srv.stats()["reserved_bytes"]
     srv.close()
-    parsed = pvvc_lib.parse_frame(frames[0])
-    need = sum(len(g) + len(c) for g, c in zip(parsed.geometry, parsed.color))
-    assert after - before >= need - (4 * 500 + 4096) and after - before < 2 * payload
+    assert need - staged <= after - before < need
