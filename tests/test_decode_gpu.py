@@ -706,3 +706,37 @@ def test_long_tier_of_a_large_batch(pvvc_lib, oracle, torch, nframes):
         a, b = one.frame_first_point[fi], one.frame_first_point[fi + 1]
         assert np.array_equal(xyz[a:b].view(np.uint32), ox.view(np.uint32)), fi
         assert rgb_matches(rgb[a:b], orgb, yuv).all(), fi
+
+
+@pytest.mark.parametrize("tune", [None, (3, 4, 32, -1, -1, 32), (3, 4, 64, -1, -1, 32), (3, 4, 128, 16, 50, 8),
+                                  (3, 4, 256, 152, 90, 16), (1, 4, 256, 4, -1, 32)])
+def test_windowed_rlgr_bit_exact(pvvc_lib, oracle, torch, tune):
+    """Very large coefficients through the windowed RLGR, with and without a long tier
+    and a medium one, for every CTA size: the first stream equals the oracle's decode,
+    the others the first."""
+    frames = _large_value_frames(pvvc_lib, 20)
+    parsed = [pvvc_lib.parse_frame(b) for b in frames]
+    one = pvvc_lib.pack_frames(parsed)
+    batch, nslots = _window_batch(pvvc_lib, torch, parsed)
+    info = pvvc_lib.Plan(batch, tune=tune).info()
+    assert info["group_ctas"] > 0 and info["singles_a"] == 0
+    # what is cleared for a per-slice RLGR: the long tier at most, a quarter of the groups
+    assert info["clear_bytes"] <= 3 * 4 * int(batch.size.astype(np.int64).sum()) * 32 // 20 // 2
+    assert (info["clear_bytes"] > 0) == (tune is None or tune[3] > 0)
+    dec = pvvc_lib.Decoder(nslots=nslots, max_leaves=4096)
+    xyz, rgb, st, p24 = decode_batch(torch, pvvc_lib, dec, batch, points24=True, tune=tune)
+    assert (st == 0).all(), np.unique(st)
+    P = one.points
+    for s in range(1, nslots // 8):
+        for a in (xyz, rgb, p24):
+            assert np.array_equal(a[s * P:(s + 1) * P].view(np.uint8), a[:P].view(np.uint8)), s
+    f = np.float32
+    for fi, (ox, orgb, ost, yuv) in enumerate(oracle_decode(oracle, pvvc_lib, frames, 16)):
+        a, b = one.frame_first_point[fi], one.frame_first_point[fi + 1]
+        assert np.array_equal(xyz[a:b].view(np.uint32), ox.view(np.uint32)), fi
+        y, u, v = yuv[:, 0], yuv[:, 1], yuv[:, 2]
+        want = np.stack([(y + f(1.402) * (v - f(128))) / f(255),
+                         ((y - f(0.3441) * (u - f(128))) - f(0.7141) * (v - f(128))) / f(255),
+                         (y + f(1.772) * (u - f(128))) / f(255)], 1).astype(np.float32)
+        assert np.array_equal(p24[a:b, 3:].view(np.uint32), want.view(np.uint32)), fi
+        assert rgb_matches(rgb[a:b], orgb, yuv).all(), fi
