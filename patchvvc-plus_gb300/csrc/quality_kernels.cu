@@ -278,7 +278,6 @@ __global__ void __launch_bounds__(kQThreads) k_q_query(QPair pr, double* __restr
         float best = FLT_MAX;
         int bi = 0x7FFFFFFF;
         auto run = [&](uint32_t row, int x0, int x1) {  // the points of cells [x0, x1] of a row
-            if (x0 > x1) return;
             const uint32_t e = __ldg(cell + row + x1 + 1);
             for (uint32_t k = __ldg(cell + row + x0); k < e; ++k) {
                 const float4 p = __ldg(sorted + k);
@@ -302,12 +301,9 @@ __global__ void __launch_bounds__(kQThreads) k_q_query(QPair pr, double* __restr
             return fmaxf(d - pad, 0.f);
         };
         // a first point from the query's own cell, or boxes of growing size; then
-        // the rows of cells inside the ball to the best one.  The box before, [ax0,
-        // ax1] and so on, is done with: a far outlier makes cells of very many
-        // points, which cost twice as much when each was gone through again (200k
-        // points in one cell: 99 ms, 48 now).
-        int ax0 = qcell(g, x, 0), ay0 = qcell(g, y, 1), az0 = qcell(g, z, 2), ax1 = ax0, ay1 = ay0, az1 = az0;
-        run(((uint32_t)az0 * g.dim[1] + ay0) * g.dim[0], ax0, ax0);
+        // the rows of cells inside the ball to the best one
+        const int cx = qcell(g, x, 0), cy = qcell(g, y, 1), cz = qcell(g, z, 2);
+        run(((uint32_t)cz * g.dim[1] + cy) * g.dim[0], cx, cx);
         float rad = 0.5f * g.h;
         for (bool last = false; !last; rad *= 4.f) {
             const bool bounded = bi != 0x7FFFFFFF;
@@ -317,19 +313,19 @@ __global__ void __launch_bounds__(kQThreads) k_q_query(QPair pr, double* __restr
                       z0 = cells(z - o, 2), z1 = cells(z + o, 2);
             last = bounded || !(rad < FLT_MAX) ||
                    (x0 == 0 && y0 == 0 && z0 == 0 && x1 == g.dim[0] - 1 && y1 == g.dim[1] - 1 && z1 == g.dim[2] - 1);
+            // the ball within the query's own cell: done.  (A far outlier makes cells of
+            // very many points, which cost twice as much when they were gone through
+            // again: 200k points in one, 99 ms, 48 now.)
+            if (bounded && x0 == x1 && y0 == y1 && z0 == z1) break;
             for (int zz = z0; zz <= z1; ++zz) {
                 const float gz = gap(zz, z, 2), gz2 = gz * gz * 0.9999f;
                 if (gz2 > best) continue;
                 for (int yy = y0; yy <= y1; ++yy) {
                     const float gy = gap(yy, y, 1);
                     if (gz2 + gy * gy * 0.9999f > best) continue;
-                    const uint32_t row = ((uint32_t)zz * g.dim[1] + yy) * g.dim[0];
-                    const bool in = zz >= az0 && zz <= az1 && yy >= ay0 && yy <= ay1;
-                    run(row, x0, in ? min(x1, ax0 - 1) : x1);
-                    if (in) run(row, max(x0, ax1 + 1), x1);
+                    run(((uint32_t)zz * g.dim[1] + yy) * g.dim[0], x0, x1);
                 }
             }
-            ax0 = x0, ax1 = x1, ay0 = y0, ay1 = y1, az0 = z0, az1 = z1;
         }
         float qc[3], tc[3];
         yuv601(c.rgb + 3ull * i, qc);
