@@ -627,8 +627,9 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
                 // a part's two level buffers: its range of every slice's last
                 // internal level (never wider than the leaves), or one whole level
                 const int seg = seg_of(gi);
-                const uint64_t parts = (uint64_t)(seg == kSegB ? p->few_parts_b : p->few_parts_a);
-                p->few_floats[seg] = std::max(p->few_floats[seg], 6 * std::max(gn, g.count * ((gn + parts - 1) / parts)));
+                const uint64_t slack = 2 * kFewSlack, parts = (uint64_t)(seg == kSegB ? p->few_parts_b : p->few_parts_a);
+                const uint64_t rows = std::max(gn + slack, g.count * ((gn + parts - 1) / parts + slack));
+                p->few_floats[seg] = std::max(p->few_floats[seg], 6 * rows);
                 continue;
             }
             c = align_up(c, 32);  // a region's rows are whole 128-byte lines (vector stores, prefetches)

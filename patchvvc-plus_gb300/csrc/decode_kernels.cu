@@ -1513,13 +1513,13 @@ __global__ void __launch_bounds__(32 * kGrpWarps, 3) k_raht_group(const SliceWor
 // lanes are as full as the level is wide, where k_raht_group's lane per slice
 // leaves 32 - count of them idle, and there are 3 n floats a slice to clear
 // instead of 96 n a group.  The level signal of the part's own nodes is
-// [slice][node][yuv] in the CTA's scratch region; a node's children that belong to
-// another part are not kept.  A part's range of a level is no wider than its range
-// of the last one unless empty nodes lie between, and then the slices go through
-// in chunks that fit.  The leaves of 32 nodes are contiguous: their colours go
-// through the warp's shared rows, then a lane writes a point.  At the last
-// internal level the intra slice, when the group has one, goes first: the others
-// read its colours.
+// [slice][node][yuv] in the CTA's scratch region, between kFewSlack rows for the
+// children of its end nodes that belong to another part.  A part's range of a
+// level is no wider than its range of the last one unless empty nodes lie between,
+// and then the slices go through in chunks that fit.  The leaves of 32 nodes are
+// contiguous: their colours go through the warp's shared rows, then a lane writes
+// a point.  At the last internal level the intra slice, when the group has one,
+// goes first: the others read its colours.
 //
 // 58 groups of 8 slices (0.8M points): k_raht_group took 275 us for its long tier
 // (22 CTAs, 8 of 32 lanes), this 36 (110 CTAs); 1,023 groups of 2 (4M points): 728
@@ -1670,7 +1670,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                 auto width = [&](int l) { return max(s_hi[l], s_lo[l]) - s_lo[l]; };
                 uint32_t widest = 0;
                 for (int l = 0; l < H - 1; ++l) widest = max(widest, width(l));
-                const size_t row = 3ull * widest;  // a slice's level signal
+                const size_t row = 3ull * (widest + 2 * kFewSlack);  // a slice's level signal
                 // slices at a time: all, but for a range widened by empty nodes (the
                 // buffers hold a slice of any width up to N, the widest level)
                 const int chunk = widest ? (int)min((uint64_t)na, scratch_floats / 2 / row) : 0;
@@ -1679,7 +1679,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                 auto nodes = [&](int l, int first, int f0, int nf, bool predict) {
                     const bool last = l == H - 2;
                     const uint32_t lo = s_lo[l], nj = width(l), nbatch = (nj + 31) / 32;
-                    const uint32_t clo = last ? 0u : s_lo[l + 1], cnj = last ? 0u : width(l + 1);
+                    const uint32_t clo = last ? 0u : s_lo[l + 1];
                     // the slices in chunks, so that every warp has two units or more
                     const int chunks = nbatch ? min(nf, (int)((2 * kFewWarps + nbatch - 1) / nbatch)) : 1;
                     const int per = (nf + chunks - 1) / max(chunks, 1);
@@ -1698,21 +1698,19 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                         const uint32_t base = __shfl_sync(0xffffffffu, rec.cb, 0);
                         const uint32_t total = __shfl_sync(0xffffffffu, rec.cb + __popc(rec.byte), nv - 1) - base;
                         for (int f = fa; f < fb; ++f) {
-                            const float* g = gA + (f - first) * row + 3ull * (j - lo);
+                            const float* g = gA + (f - first) * row + 3ull * (j + kFewSlack - lo);
                             float oy[8], ou[8], ov[8];
                             lane_inverse(rec, coef + s_coef[f], N, g[0], g[1], g[2], oy, ou, ov);
                             if (!last) {
-                                float* const gb = gB + (f - first) * row;
-                                uint32_t at = rec.cb - clo;  // (unsigned: children before the range are beyond it)
+                                float* gb = gB + (f - first) * row;
+                                gb += 3ull * (rec.cb + kFewSlack - clo);
 #pragma unroll
                                 for (int c = 0; c < 8; ++c) {
                                     if (!(rec.byte & (0x80u >> c))) continue;
-                                    if (at < cnj) {
-                                        gb[3ull * at] = oy[c];
-                                        gb[3ull * at + 1] = ou[c];
-                                        gb[3ull * at + 2] = ov[c];
-                                    }
-                                    ++at;
+                                    gb[0] = oy[c];
+                                    gb[1] = ou[c];
+                                    gb[2] = ov[c];
+                                    gb += 3;
                                 }
                                 continue;
                             }
@@ -1740,7 +1738,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) k_raht_few(const SliceWork* __
                     gB = bufB;
                     if (tid < nf) {
                         const float* cy = coef + s_coef[first + tid];
-                        float* g = gA + tid * row;
+                        float* g = gA + tid * row + 3 * kFewSlack;
                         g[0] = cy[0];
                         g[1] = cy[N];
                         g[2] = cy[2ull * N];

@@ -27,6 +27,7 @@ constexpr int kWinGroupsPerLongCta = 4;
 // In a batch with window groups, groups of fewer slices are inverse-transformed
 // by k_raht_few, the others by k_raht_group; in any other batch all by k_raht_few.
 constexpr int kFewBelow = 16;
+constexpr uint32_t kFewSlack = 7;  // a node's children beside the one in a part's range
 // The long tier's groups go to k_raht_few as well, whatever their size: it splits
 // each over several CTAs, a shorter tail for more instructions a point.  That pays
 // while the other groups do not fill the device beside it, below kLongWidePerSm
