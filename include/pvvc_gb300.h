@@ -94,11 +94,11 @@ int pvvc_plan_query(const pvvc_plan* plan, uint64_t* total_points, uint64_t* wor
  * (src/cuda/render/render.cc:269-301, block = 1).
  *
  * RLGR runs in one of two forms.  Groups of at least 16 slices of one slot,
- * all of one size (the frames of a patch in a GoP), form size tiers of whole
- * groups: the long tier is decoded one thread per slice into planes cleared
- * beforehand, the medium and short tiers one warp per group, each warp
- * staging its coefficients in a shared-memory window and writing them as
- * whole lines (no plane clear).  Every other slice is decoded one thread per
+ * all of one size (the frames of a patch in a GoP), if there are as many as the
+ * device has SMs, form size tiers of whole groups: the long tier is decoded
+ * one thread per slice into planes cleared beforehand, the medium and short
+ * tiers one warp per group, each warp staging its coefficients in a
+ * shared-memory window and writing them as whole lines (no plane clear).  Every other slice is decoded one thread per
  * slice into planes cleared beforehand; when no group qualifies, those
  * slices are split into the size tiers below. */
 typedef struct {
@@ -244,7 +244,8 @@ int pvvc_host_stage_times(double* out, int32_t n);
  * libzstd rejects; it is stricter in one place (a Huffman literal stream must
  * end exactly on its first bit, which libzstd's fast 4-stream path does not
  * check).  Arrays are device memory; out_len may be NULL.  One warp per job;
- * stream-ordered.  The reference sizes dst by the first frame's declared
+ * stream-ordered.  A source is read by whole aligned 4-byte words, up to three
+ * bytes before its first and after its last (they are not used).  The reference sizes dst by the first frame's declared
  * content size: pvvc_zstd_content_size reads it on the host. */
 int pvvc_zstd_inflate_batch(int32_t njobs, const uint8_t* src, const uint64_t* src_off, const uint32_t* src_len,
                             uint8_t* dst, const uint64_t* dst_off, const uint32_t* dst_cap, uint32_t* out_len,

@@ -491,8 +491,9 @@ int build_plan(const pvvc_batch_desc* d, pvvc_plan* p, const pvvc_tune* tune, cu
             return (int32_t)(v.end() - std::stable_partition(v.begin(), v.end(), [&](const GroupDesc& g) { return !is_few(g); }));
         };
         // Window groups (while there are enough, as above): phase-A groups of at
-        // least kWinGroupMin slices, all of one size, in size tiers of whole groups (ga is already largest
-        // first), so a tier's inverse RAHT waits for its own RLGR only.  The
+        // least kWinGroupMin slices, all of one size, in size tiers of whole groups
+        // (ga is already largest first), so a tier's inverse RAHT waits for its own
+        // RLGR only.  The
         // long tier's slices -- the critical path -- are decoded by the
         // per-slice long launch, whose iterations are the cheapest, into
         // planes cleared first; the medium and short tiers by the windowed

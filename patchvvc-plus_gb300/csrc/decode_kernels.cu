@@ -284,14 +284,13 @@ __global__ void __launch_bounds__(T) k_tree(const SliceWork* __restrict__ work, 
 // owns a ring of kRing blocks (kRing * 16 bytes, aligned to its size), filled
 // by cp.async.  The copies are requested at a point the whole warp passes
 // together (stage(), every kRlCheck iterations: as many blocks as those can
-// take),
-// never from inside a lane's own branch: with 32 slices in a warp, some lane
-// needs a block in nearly every iteration, and each such branch cost the warp
-// its instructions and a wait for copies that other lanes had just requested.  `landed` counts the blocks
-// known to be in shared memory: those requested three stage() calls ago.  A
-// lane that may run out of landed words before the next stage() -- only after
-// codes longer than 32 bits -- refills its ring synchronously.  Blocks past
-// the payload are zero.
+// take), never from inside a lane's own branch: with 32 slices in a warp, some
+// lane needs a block in nearly every iteration, and each such branch cost the
+// warp its instructions and a wait for copies that other lanes had just
+// requested.  `landed` counts the blocks known to be in shared memory: those
+// requested three stage() calls ago.  A lane that may run out of landed words
+// before the next stage() -- only after codes longer than 32 bits -- refills its
+// ring synchronously.  Blocks past the payload are zero.
 constexpr int kRing = 8;             // 16-byte blocks per lane
 constexpr uint32_t kRlCheck = 8;     // iterations between stage() calls (4: 5-10% slower, 16: no faster);
                                      // a fast iteration takes at most one word
@@ -1841,14 +1840,14 @@ cudaError_t launch_tree(const SliceWork* work, int nintra, const uint8_t* payloa
     return cudaGetLastError();
 }
 
-// smem: dynamic shared memory reserved per CTA (unused by the kernel; it
-// limits which CTAs share an SM, see kRlgrLongSmem)
 cudaError_t launch_refresh(SliceWork* work, int n, const CallFields& f, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     k_refresh<<<(n + 255) / 256, 256, 0, s>>>(work, n, f);
     return cudaGetLastError();
 }
 
+// smem: dynamic shared memory reserved per CTA (beyond the payload rings it
+// limits which CTAs share an SM, see kRlgrLongSmem)
 cudaError_t launch_rlgr(const SliceWork* work, const int32_t* order, int nslices, const uint8_t* payload, float* coef,
                         int32_t* rstatus, int block, int smem, cudaStream_t s) {
     if (nslices <= 0) return cudaSuccess;
@@ -1882,7 +1881,7 @@ cudaError_t launch_rlgr_long(const SliceWork* work, const int32_t* order, int ns
 }
 
 // Windowed RLGR of `ngroups` groups, one warp each, `warps` per CTA; a
-// warp's rings and window take 10 KB, a CTA at least kWinMinSmem, more than
+// warp's rings and window take 12 KB, a CTA at least kWinMinSmem, more than
 // the SM of a long per-slice CTA has left.
 cudaError_t launch_rlgr_win(const SliceWork* work, const GroupDesc* groups, int ngroups, const int32_t* items,
                             const uint8_t* payload, float* coef, int32_t* rstatus, int warps, cudaStream_t s) {

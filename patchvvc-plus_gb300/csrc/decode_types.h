@@ -11,7 +11,7 @@ constexpr int kMaxLevels = 32;  // octree height limit (the header stores a u8)
 // One slice in the work queue (queue order = intra first, then by size).
 // RLGR launches split by slice length: a CTA of the long-slice launch (128
 // threads, one warp per scheduler) reserves this much dynamic shared memory,
-// which no RLGR code uses, so that no other CTA fits on its SM -- neither one
+// far more than its payload rings, so that no other CTA fits on its SM -- neither one
 // of the other RLGR launch (kRlgrShortSmem each) nor one of the grouped
 // inverse RAHT (~20 KB) that runs beside it.  The serial bit chains of the
 // longest slices then run without sharing issue slots, while the rest of the

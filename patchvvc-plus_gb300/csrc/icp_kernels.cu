@@ -44,6 +44,7 @@ constexpr int kMaxCells = 16384;
 constexpr int kGridSmem = 4 * (kMaxCells + 1);
 constexpr int kIcpCellMul = 2;      // cells per target point, pvvc_icp_batch / pvvc_cloud_mse_batch
 constexpr int kNoAllocCellMul = 2;  // cells per target point, pvvc_icp_batch_noalloc
+static_assert(kNoAllocCellMul == kIcpCellMul, "k_icp finds both entry points' cell arrays by kIcpCellMul");
 __host__ __device__ __forceinline__ int cell_budget(int kmul, uint32_t n) {
     const long long c = (long long)kmul * n;
     return (int)(c < 64 ? 64 : (c > kMaxCells ? kMaxCells : c));
@@ -1063,7 +1064,6 @@ extern "C" int pvvc_icp_batch(int32_t npairs, const float* src_xyz, const uint32
     cudaStream_t s = (cudaStream_t)stream;
     if (!grid_attr_ready()) return PVVC_ERR_CUDA;
     k_grid<256><<<npairs, 256, kGridSmem, s>>>(tgt_xyz, tgt_off, nullptr, w.hdr, w.cstart, w.sorted, kIcpCellMul);
-    // the source-side grid's place (pvvc_cloud_mse_batch's) holds the neighbours
     // the source-side grid's place (pvvc_cloud_mse_batch's) holds the neighbours
     const uint32_t nsrc = (uint32_t)std::min<uint64_t>(total_src_points, 0xFFFFFFFFu);
     auto launch = [&](auto kernel, int threads) {

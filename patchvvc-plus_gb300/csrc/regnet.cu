@@ -182,8 +182,10 @@ __global__ void __launch_bounds__(256) k_sample_l1(int npairs, const int32_t* __
 
 // X1 and its transpose from given x0 rows (the gradient-check entry), 256 rows a
 // block, both written in whole lines through shared memory: layer 2's weight
-// gradient reads the transpose (blocks of [channel][64 rows]).  For 524,288 rows 41 us with a row a thread and
-// 42 more for a transpose kernel; 25 now (134 MB written).
+// gradient reads the transpose (blocks of [channel][64 rows]).  For 524,288 rows
+// 41 us with a row a thread and 42 more for a transpose kernel; 25 now (134 MB
+// written).  (k_sample_l1 writes the transpose a row a thread, by two-byte stores:
+// 71 us, 41.5 without it.)
 constexpr int kL1Row = kD1 / 2 + 1;  // words of a staged row: odd, so that a column's words spread over the banks
 __global__ void __launch_bounds__(256) k_l1(int64_t rows, const float* __restrict__ x0, const float* __restrict__ w1,
                                             const float* __restrict__ b1, __nv_bfloat16* __restrict__ x1,
@@ -407,9 +409,10 @@ __global__ void __launch_bounds__(kD2) k_pool_bwd_w3(int nclouds, const float* _
 // outputs are summed over its bucket in channel order and written at once,
 // zero rows included: a warp takes 16 rows of each half, a lane four columns,
 // eight rows' X2 in flight.  The block also writes its part of dY2's transpose
-// (dY2T, blocks of [channel][64 rows], for the weight gradient) and its column sums (for db2) from the rows in shared memory,
-// instead of kernels that read dY2 again: 1,024 pairs took 117 us and 85 more for
-// the transpose; 113 now (402 MB read and written).
+// (dY2T, blocks of [channel][64 rows], for the weight gradient) and its column
+// sums (for db2) from the rows in shared memory, instead of kernels that read dY2
+// again: 1,024 pairs took 117 us and 85 more for the transpose; 113 now (402 MB
+// read and written).
 constexpr int kDyRow = kD2 + 2;  // staged row of dY2 (bf16): 65 words, odd
 __global__ void __launch_bounds__(256, 4) k_pool_bwd_x2(const float* __restrict__ dh0, const __nv_bfloat16* __restrict__ h0,
                                                     const int32_t* __restrict__ amax, const __nv_bfloat16* __restrict__ w3,
