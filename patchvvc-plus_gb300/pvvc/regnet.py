@@ -84,7 +84,8 @@ class RegNet:
 
     def grad(self, x0, y, lambda_w: float, stream: int = 0):
         """Gradient and loss for normalised inputs x0 (device [B,2,P,3] fp32)
-        and targets y (device [B,6]); no update.  Returns device tensors."""
+        and targets y (device [B,6]), B a multiple of 64; no update.  Returns
+        device tensors."""
         import torch
         B = int(y.shape[0])
         g = torch.empty(self.nparam, dtype=torch.float32, device=y.device)
@@ -94,7 +95,8 @@ class RegNet:
         return g, loss
 
     def train_step(self, data: "PairData", ids, seed: int, opt: AdamW, loss_out=None, stream: int = 0) -> None:
-        """One AdamW step on pairs `ids` (device int32) of a labelled dataset."""
+        """One AdamW step on pairs `ids` (device int32, a multiple of 64 of them) of
+        a labelled dataset."""
         L.check(L.lib().pvvc_regnet_train_step(self.h, int(ids.numel()), ids.data_ptr(), data.src.data_ptr(),
                                                data.soff.data_ptr(), data.tgt.data_ptr(), data.toff.data_ptr(),
                                                data.T_label.data_ptr(), data.omega_label.data_ptr(), seed, C.byref(opt),
